@@ -55,7 +55,11 @@ extern "C" {
 #define VT_REDUCE_VOLUME 3
 
 /* ---- walk kernels ------------------------------------------------------ */
-#define VT_KERNEL_AUTO 0        /* THREAD_FP32; BATCHED below 65,536 rays       */
+#define VT_KERNEL_AUTO 0        /* one ray per thread on neighbour lists built  */
+                                /* on first need; before that, on periodic      */
+                                /* clouds and on trees with leaves of more than */
+                                /* 8 points: THREAD_FP32, BATCHED below 65,536  */
+                                /* rays, or the autotuner's choice              */
 #define VT_KERNEL_PLAIN_FP64 1  /* one ray per thread in the caller's order,    */
                                 /* full-FP64 k-NN from the root                 */
 #define VT_KERNEL_BATCHED 2     /* persistent queue, one warp per ray,          */

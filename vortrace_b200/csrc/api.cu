@@ -94,10 +94,29 @@ int vt::check_projectable(const vt_cloud* cl, int mode) {
 // vt_cloud_autotune replaces the rule by its measured choice for batches of
 // at least its sample's size.
 constexpr uint64_t kThreadKernelMinRays = 65536;
-int vt::resolve_kernel(const vt_cloud* cl, int kernel, uint64_t nrays) {
-  if (kernel != VT_KERNEL_AUTO) return kernel;
+int vt::resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays) {
   if (cl->tuned_kernel != VT_KERNEL_AUTO && nrays >= cl->tuned_min_rays) return cl->tuned_kernel;
   return nrays < kThreadKernelMinRays ? VT_KERNEL_BATCHED : VT_KERNEL_THREAD_FP32;
+}
+
+// The list walk (listed.cuh) takes every AUTO launch once the neighbour lists
+// are built, whatever the autotuner chose among the tree kernels (4.2 times
+// faster at 1M rays, twice at 300).  Building them costs about 3 ns a point and
+// the allocation of 1 KB a point (2M points: 7 ms), a crossing on the tree 0.9 ns
+// (1M rays) to 6 ns (16,384 rays), so they are built when the crossings walked on
+// the cloud without them, 1.5 cube roots of n a ray, reach the number of points:
+// a cloud that sees a few rays never pays for them.
+constexpr double kNbrCrossingsPerPoint = 1.0;
+int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
+  if (kernel != VT_KERNEL_AUTO) return kernel == kKernelList ? VT_KERNEL_BATCHED_FP64 : kernel;
+  if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64) {
+    cl->nbr_credit += 1.5 * std::cbrt((double)cl->npart) * (double)nrays;
+    if (cl->nbr_credit >= kNbrCrossingsPerPoint * (double)cl->npart) {
+      const int rc = build_nbr_lists(cl);
+      if (rc) return resolve_tree_kernel(cl, nrays);
+    }
+  }
+  return cl->view.nbr ? kKernelList : resolve_tree_kernel(cl, nrays);
 }
 
 static cudaStream_t pick_stream(vt_cloud* cl, void* s) {
@@ -422,7 +441,8 @@ int vt_cloud_get_info(const vt_cloud* cl, vt_cloud_info* info) {
   info->tree_build_ms = cl->build_ms;
   info->device_bytes = cl->pts_d.bytes() + cl->pts32_d.bytes() + cl->nodes_d.bytes() +
                        cl->nodes32_d.bytes() + cl->perm_d.bytes() + cl->fields_d.bytes() +
-                       cl->boxlo_d.bytes() + cl->boxhi_d.bytes() + cl->leaf32_d.bytes() + cl->tt_nodes_d.bytes() +
+                       cl->boxlo_d.bytes() + cl->boxhi_d.bytes() + cl->leaf32_d.bytes() + cl->nbr_d.bytes() +
+                       cl->nbr_hdr_d.bytes() + cl->tt_nodes_d.bytes() +
                        cl->tt_pts_d.bytes() + cl->tt_tid_d.bytes();
   info->tie_tree_nodes = cl->view.tt_nodes ? cl->tt_nodes_d.n : 0;
   info->tie_tree_depth = cl->view.tt_nodes ? cl->tt_depth : 0;
@@ -463,6 +483,7 @@ int vt_knn(const vt_cloud* ccl, const double* q, uint64_t nq, int k, int64_t* id
   VT_GUARD_END
 }
 
+// `kernel`: as resolve_kernel gives it
 static int project_device_locked(vt_cloud* cl, const double* d_starts, const double* d_ends,
                                  uint64_t nrays, int mode, int kernel, double* d_out,
                                  cudaStream_t st, vt_stats* stats, int out_kind,
@@ -474,7 +495,7 @@ static int project_device_locked(vt_cloud* cl, const double* d_starts, const dou
   io.nout = mode == VT_REDUCE_VOLUME ? 3 : (int)cl->nfields;
   io.out = d_out;
   io.counts = d_counts;
-  return vt::run_walk(cl, io, out_kind, mode, resolve_kernel(cl, kernel, io.nrays), st, stats);
+  return vt::run_walk(cl, io, out_kind, mode, kernel, st, stats);
 }
 
 int vt_project_device(vt_cloud* cl, const double* d_starts, const double* d_ends,
@@ -487,8 +508,9 @@ int vt_project_device(vt_cloud* cl, const double* d_starts, const double* d_ends
   VT_CUDA(cudaSetDevice(cl->device));
   if (stats) memset(stats, 0, sizeof(*stats));
   if (nrays == 0) return VT_OK;
-  return project_device_locked(cl, d_starts, d_ends, nrays, mode, kernel, d_out,
-                               pick_stream(cl, stream), stats, vt::kOutImage, nullptr);
+  return project_device_locked(cl, d_starts, d_ends, nrays, mode,
+                               resolve_kernel(cl, kernel, nrays), d_out, pick_stream(cl, stream),
+                               stats, vt::kOutImage, nullptr);
   VT_GUARD_END
 }
 
@@ -512,8 +534,9 @@ int vt_project(vt_cloud* cl, const double* starts, const double* ends, uint64_t 
                           cudaMemcpyHostToDevice, st));
   VT_CUDA(cudaMemcpyAsync(cl->ws_ends.p, ends, 3 * nrays * sizeof(double),
                           cudaMemcpyHostToDevice, st));
-  rc = project_device_locked(cl, cl->ws_starts.p, cl->ws_ends.p, nrays, mode, kernel,
-                             cl->ws_out.p, st, stats, vt::kOutImage, nullptr);
+  rc = project_device_locked(cl, cl->ws_starts.p, cl->ws_ends.p, nrays, mode,
+                             resolve_kernel(cl, kernel, nrays), cl->ws_out.p, st, stats,
+                             vt::kOutImage, nullptr);
   if (rc) return rc;
   VT_CUDA(cudaMemcpyAsync(out, cl->ws_out.p, nrays * nout * sizeof(double),
                           cudaMemcpyDeviceToHost, st));
@@ -571,8 +594,9 @@ int vt_project_grid(vt_cloud* cl, const double extent[4], uint64_t nx, uint64_t 
   cudaStream_t st = cl->stream;
   if ((rc = vt::launch_grid_rays(extent, nx, ny, bounds, cl->ws_starts.p, cl->ws_ends.p, st)))
     return rc;
-  rc = project_device_locked(cl, cl->ws_starts.p, cl->ws_ends.p, nrays, mode, kernel,
-                             cl->ws_out.p, st, stats, vt::kOutImage, nullptr);
+  rc = project_device_locked(cl, cl->ws_starts.p, cl->ws_ends.p, nrays, mode,
+                             resolve_kernel(cl, kernel, nrays), cl->ws_out.p, st, stats,
+                             vt::kOutImage, nullptr);
   if (rc) return rc;
   VT_CUDA(cudaMemcpyAsync(out, cl->ws_out.p, nrays * nout * sizeof(double),
                           cudaMemcpyDeviceToHost, st));
@@ -621,8 +645,9 @@ int vt_project_batch(vt_cloud* cl, const vt_grid_desc* grids, uint64_t ngrids,
     VT_CUDA(cudaMemcpyAsync(cl->ws_ends.p + 3 * at, ends, 3 * nrays * sizeof(double),
                             cudaMemcpyHostToDevice, st));
   }
-  rc = project_device_locked(cl, cl->ws_starts.p, cl->ws_ends.p, total, mode, kernel,
-                             cl->ws_out.p, st, stats, vt::kOutImage, nullptr);
+  rc = project_device_locked(cl, cl->ws_starts.p, cl->ws_ends.p, total, mode,
+                             resolve_kernel(cl, kernel, total), cl->ws_out.p, st, stats,
+                             vt::kOutImage, nullptr);
   if (rc) return rc;
   VT_CUDA(cudaMemcpyAsync(out, cl->ws_out.p, total * nout * sizeof(double),
                           cudaMemcpyDeviceToHost, st));

@@ -71,6 +71,9 @@ constexpr int kTieMaxDepth = 96;
 #define VT_LEAF_SLOTS 8
 #endif
 constexpr int kLeafSlots = VT_LEAF_SLOTS;
+// neighbours kept per point, in two parts of whole groups of four
+constexpr int kNbrMax = 60;
+constexpr int kNbrGroups = 16;
 
 struct DevCloud {
   const double4* __restrict__ pts;
@@ -84,6 +87,10 @@ struct DevCloud {
   // packed sum q + (-p); NULL when a leaf holds more points
   const float4* __restrict__ leaf32;
   const double* __restrict__ fields;
+  // neighbour lists (nbrlist.cu): kNbrGroups 64-byte groups per point and a
+  // header each; NULL until they are built
+  const float4* __restrict__ nbr;
+  const uint32_t* __restrict__ nbr_hdr;
   // tight FP32 boxes (of the pts32 values) of every heap node, internal
   // nodes first then leaves: node i in [0, 2L-1)
   const float4* __restrict__ boxlo;

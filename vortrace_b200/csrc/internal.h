@@ -12,6 +12,7 @@
 
 #include "../../include/vortrace_b200.h"
 #include "common.cuh"
+#include "walkio.h"
 
 namespace vt {
 
@@ -120,6 +121,9 @@ struct vt_cloud {
   vt::DevBuf<double> fields_d;
   vt::DevBuf<float4> boxlo_d, boxhi_d;
   vt::DevBuf<float4> leaf32_d;  // SoA leaf blocks (common.cuh)
+  vt::DevBuf<float4> nbr_d;     // neighbour lists (nbrlist.cu) ...
+  vt::DevBuf<uint32_t> nbr_hdr_d;
+  double nbr_credit = 0.0;      // ... and the crossings walked without them
   // reference-order tree (tietree.cu), built when an exact tie needs it
   vt::DevBuf<vt::TieNode> tt_nodes_d;
   vt::DevBuf<double4> tt_pts_d;
@@ -138,6 +142,7 @@ struct vt_cloud {
   vt::DevBuf<vt::DevStats> ws_stats;
   vt::DevBuf<uint8_t> ws_tmp;
   vt::DevBuf<uint8_t> ws_order;  // ray sort keys, order and CUB scratch
+  vt::DevBuf<vt::WalkRec> ws_rec;  // boundaries of the list walk
 };
 
 // Segment tape of one 'integrate' or 'volume' forward
@@ -165,6 +170,14 @@ int build_tree_device(vt_cloud* cl);
 // and free (the device tree was rebuilt or reloaded)
 int build_tie_tree(vt_cloud* cl, cudaStream_t st);
 void drop_tie_tree(vt_cloud* cl);
+// neighbour lists (nbrlist.cu): build (no-op when built or when they do not
+// fit) and free (the tree was rebuilt or reloaded)
+int build_nbr_lists(vt_cloud* cl);
+void drop_nbr_lists(vt_cloud* cl);
+// the list walk (listed.cuh); chosen by resolve_kernel only
+constexpr int kKernelList = -1;
+// threads and boundaries per thread of its launch over nrays rays
+int list_scratch(const vt_cloud* cl, int64_t nrays, int64_t& threads, int& cap);
 // saved trees (tree_build.cu)
 uint64_t tree_blob_size(const vt_cloud* cl);
 int save_tree_blob(vt_cloud* cl, void* buf);
@@ -173,7 +186,10 @@ int upload_fields(vt_cloud* cl, const double* src, bool src_device, cudaStream_t
 // tree built, mode valid, volume needs valid RGBA (src/reduction.cpp:59-66)
 int check_projectable(const vt_cloud* cl, int mode);
 // the kernel VT_KERNEL_AUTO stands for with this cloud and batch size
-int resolve_kernel(const vt_cloud* cl, int kernel, uint64_t nrays);
+// (builds the neighbour lists when they are due)
+int resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays);
+// the same without the list walk
+int resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays);
 // resident blocks per SM the launch bounds of the walk kernel that runs a
 // launch of nrays rays are compiled for (VT_KERNEL_THREAD_FP32,
 // _BATCHED_FP64, _BATCHED on the current device; 0 for the others)

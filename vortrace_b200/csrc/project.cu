@@ -524,9 +524,31 @@ static int sort_rays(vt_cloud* cl, WalkIO& io, cudaStream_t st) {
   return sort_rays_into(cl->view, io, cl->ws_order.p, total, cub_bytes, st);
 }
 
+// Four times the crossings of a ray through a homogeneous cloud; a longer ray
+// goes on with tree queries.
+int list_scratch(const vt_cloud* cl, int64_t nrays, int64_t& threads, int& cap) {
+  int dev = 0, nsms = 0;
+  VT_CUDA(cudaGetDevice(&dev));
+  VT_CUDA(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev));
+  threads = list_blocks(nrays, nsms) * kListBlock;
+  const int want = (int)(4.0 * std::cbrt((double)cl->npart)) & ~63;
+  cap = want < 256 ? 256 : (want > 2048 ? 2048 : want);
+  return VT_OK;
+}
+
 // Walk launch with the handle's (grow-only) workspace as scratch.
 int run_walk(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel, cudaStream_t st,
              vt_stats* stats) {
+  if (kernel == kKernelList) {
+    int64_t threads = 0;
+    const int rc = list_scratch(cl, io.nrays, threads, io.rec_cap);
+    if (rc) return rc;
+    if (cl->ws_rec.reserve((size_t)threads * io.rec_cap)) {
+      cudaGetLastError();  // no memory for the boundaries: walk on the tree
+      kernel = resolve_tree_kernel(cl, io.nrays);
+    }
+    io.rec = cl->ws_rec.p;
+  }
   if (kernel != VT_KERNEL_PLAIN_FP64 && !cl->periodic) {
     const int rc = sort_rays(cl, io, st);
     if (rc) return rc;
@@ -583,8 +605,10 @@ struct vt_graph {
   vt::DevBuf<int> stack_id;
   vt::DevBuf<double> stack_s;
   vt::DevBuf<uint8_t> order;
+  vt::DevBuf<vt::WalkRec> rec;
   vt::WalkIO io{};
   int mode = 0;
+  uint64_t tree_gen = 0;  // the cloud's tree (and lists) at capture time
   const double4* pts = nullptr;  // the cloud's buffers at capture time
   const double* fields = nullptr;
   ~vt_graph() {
@@ -628,7 +652,16 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
     io.gstack_s = g->stack_s.p;
     io.gstack_cap = cl->stack_cap;
     io.slow_threads = slow_threads;
-    const int k = resolve_kernel(cl, kernel, nrays);
+    int k = resolve_kernel(cl, kernel, nrays);
+    if (k == kKernelList) {
+      int64_t threads = 0;
+      if ((rc = list_scratch(cl, io.nrays, threads, io.rec_cap))) return rc;
+      if (g->rec.alloc((size_t)threads * io.rec_cap)) {
+        cudaGetLastError();
+        k = resolve_tree_kernel(cl, nrays);
+      }
+      io.rec = g->rec.p;
+    }
     size_t total = 0, cub_bytes = 0;
     if (k != VT_KERNEL_PLAIN_FP64 && !cl->periodic) {
       if ((rc = sort_rays_bytes(io.nrays, total, cub_bytes))) return rc;
@@ -653,6 +686,7 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
     }
     g->graph = graph;
     VT_CUDA(cudaGraphInstantiate(&g->exec, graph, 0));
+    g->tree_gen = cl->tree_gen;
     g->pts = cl->view.pts;
     g->fields = cl->view.fields;
     *out = g.release();
@@ -665,7 +699,8 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
 int vt_graph_launch(vt_graph* g, void* stream) {
   using namespace vt;
   if (!g) return set_error(VT_ERR_INVALID, "null graph handle");
-  if (g->cl->view.pts != g->pts || g->cl->view.fields != g->fields)
+  if (g->cl->view.pts != g->pts || g->cl->view.fields != g->fields ||
+      g->cl->tree_gen != g->tree_gen)
     return set_error(VT_ERR_RUNTIME,
                      "the cloud's tree or fields were reallocated after the graph was created");
   VT_CUDA(cudaSetDevice(g->device));

@@ -391,6 +391,8 @@ static int finish_tree(vt_cloud* cl, int depth, const double lo[3], const double
   double mext = 0.0;
   for (int j = 0; j < 3; ++j) mext = fmax(mext, fmax(fabs(hi[j] - org[j]), fabs(lo[j] - org[j])));
 
+  drop_nbr_lists(cl);
+  cl->nbr_credit = 0.0;
   cl->perm_d = std::move(pa);
   cl->pts_d = std::move(pts);
   cl->pts32_d = std::move(pts32);

@@ -390,6 +390,8 @@ __global__ void __launch_bounds__(128) k_slow(DevCloud c, WalkIO io) {
 // with warp-cooperative search (warp.cuh)
 #include "batched.cuh"
 #include "warp.cuh"
+// one ray per thread on the neighbour lists
+#include "listed.cuh"
 
 namespace vt {
 
@@ -403,6 +405,9 @@ int launch_walk_t(vt_cloud* cl, WalkIO& io, int kernel, cudaStream_t st) {
       // second pass over the rays deferred for the reference-order tree
     } else if (cl->periodic) {
       k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
+    } else if (kernel == kKernelList) {
+      const int rc = launch_list<MODE, NF, OUT>(cl, io, st);
+      if (rc) return rc;
     } else if (kernel == VT_KERNEL_PLAIN_FP64) {
       k_plain<MODE, NF, OUT, false><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
     } else if (kernel == VT_KERNEL_BATCHED && cl->nfields <= 32) {

@@ -36,6 +36,16 @@ constexpr int kErrNonFinite = 16;
 
 struct WalkDiag;
 
+// One cell of a marched ray (listed.cuh): the parameter t of the boundary into
+// it, the parameter a of its generator's foot on the ray, the foot's squared
+// distance q from the generator, and the rate at which the squared distances to
+// the boundary's two cells part along the ray (0: not certified).  One sector.
+struct __align__(32) WalkRec {
+  double t, a, q;
+  int32_t cell;
+  float slope;
+};
+
 struct WalkIO {
   const double* starts;  // nrays x 3, device
   const double* ends;    // nrays x 3, device
@@ -63,6 +73,9 @@ struct WalkIO {
   void* tape;            // kOutTape: entries [0, tape_cap) (TapeEntry, or TapeEntryV for volume)
   unsigned long long* tape_count;  // kOutTape: entries appended (may exceed tape_cap)
   unsigned long long tape_cap;
+  WalkRec* rec;          // list walk: rec_cap boundaries per thread (NULL: not this kernel)
+  int rec_cap;
+  int batch;             // list walk: rays a warp takes at a time (1..32)
   WalkDiag* diag;
   int deferred;          // k_slow only, over the entries deferred for the
                          // reference-order tree (which is now built)
