@@ -16,7 +16,7 @@
 //           every split point falls on one recorded cell, clear of its
 //           neighbours, the reference's walk is the marched sequence, and the
 //           ray is reduced from it with the reference's FP64 split points;
-//   walk    for the other rays (0.4% on clustered_2m) the reference's own loop
+//   walk    for the other rays (0.1% on clustered_2m) the reference's own loop
 //           with FP64 queries on the tree, except where certified boundaries
 //           give the answer.
 //
@@ -45,8 +45,9 @@
 // this kernel takes 69 (clustered_2m, 512x512), and is bound by the latency of
 // dependent loads (8.6 of 13.4 cycles between two instructions of a warp): the
 // lists (1 KB per point) and the records outgrow the L2.  Walk launch, tree
-// search -> lists: clustered_2m 1024x1024 171.6 -> 35.5 ms, uniform_100k 128x128
-// 6.3 -> 0.77 ms, batched_1m 569 -> 191 ms.
+// search -> lists: clustered_2m 1024x1024 171.6 -> 30.8 ms (march with its queries
+// 20 ms, replay and walk 7, reduction 4.5), uniform_100k 128x128 6.3 -> 0.67 ms,
+// batched_1m 569 -> 166 ms (10 queries a ray outside the cloud).
 #pragma once
 
 namespace vt {
@@ -107,20 +108,17 @@ __device__ __forceinline__ bool list_settle(const DevCloud& c, const RayGeom& g,
   const double4 P = ldg_pt(&c.pts[cell]);
   double a, q, e[3];
   foot(g, P, a, q, e);
-  float slope = 0.f;
   if (i > 0) {
     const double da = a - m.a;
     m.t = 0.5 * ((a + m.a) + (q - m.q) / da);
     // (bisectors within the parallel tolerance of the ray are not certified)
-    slope = __double2float_rd(2.0 * da);
-    if (!(slope > 1e-10f) || !clean) {
-      slope = 0.f;
-      m.all = false;
-    }
+    clean = clean && da > 5e-11;
+    m.all = m.all && clean;
   }
   m.a = a;
   m.q = q;
-  rec[i] = WalkRec{m.t, a, q, cell, slope};
+  const float qf = (float)q;
+  rec[i] = WalkRec{a, clean ? qf : -qf, cell};
   const double ta = m.t - a;
   w[0] = (float)fma(ta, g.d[0], -e[0]);
   w[1] = (float)fma(ta, g.d[1], -e[1]);
@@ -285,50 +283,95 @@ __device__ __forceinline__ int list_step(const DevCloud& c, const RayGeom& g, do
   return kMarchOn;
 }
 
-// Largest index m in [lo, hi] with rec[m].t < s (lo when there is none).
-__device__ __forceinline__ int list_find(const WalkRec* rec, int lo, int hi,
-                                         double s) {
-  while (lo < hi) {
+// f_(i)(s) - f_(j)(s), f the squared distance from the ray's point s to the cells'
+// generators; `err` grows by the rounding of the FP32 offsets.
+__device__ __forceinline__ double line_diff(double ai, float qi, double aj, float qj, double s,
+                                            float& err) {
+  qi = fabsf(qi);
+  qj = fabsf(qj);
+  err = fmaf(1.3e-7f, qi + qj, err);
+  return fma(aj - ai, 2.0 * s - ai - aj, (double)qi - (double)qj);
+}
+
+// Where the lines of cells i and j (records) cross.
+__device__ __forceinline__ double line_cross(double ai, float qi, double aj, float qj) {
+  return 0.5 * ((ai + aj) + ((double)fabsf(qj) - (double)fabsf(qi)) / (aj - ai));
+}
+
+// Whether the record arrays A (foot parameters) and Q give one cell m of (i, j) as
+// the nearest at the crossing s of cells i and j, clear of its two neighbours in the
+// sequence by more than `gap` in squared distance; m receives it.
+template <class FA, class FQ>
+__device__ __forceinline__ bool list_nearest(const FA& A, const FQ& Q, int i, int j, double s,
+                                             double gap, int& m) {
+  int lo = i + 1, hi = j - 1;
+  while (lo < hi) {  // the last foot up to s, then the lowest line around it
     const int mid = (lo + hi + 1) >> 1;
-    if (rec[mid].t < s) lo = mid;
+    if (A(mid) <= s) lo = mid;
     else hi = mid - 1;
   }
-  return lo;
+  float err = 1.3e-7f * (fabsf(Q(i)) + fabsf(Q(j)));
+  float none = 0.f;
+  double am = A(lo);
+  float qm = Q(lo);
+  for (; lo + 1 < j; ++lo) {
+    const double an = A(lo + 1);
+    const float qn = Q(lo + 1);
+    if (line_diff(an, qn, am, qm, s, none) >= 0.0) break;
+    am = an;
+    qm = qn;
+  }
+  for (; lo - 1 > i; --lo) {
+    const double an = A(lo - 1);
+    const float qn = Q(lo - 1);
+    if (line_diff(an, qn, am, qm, s, none) >= 0.0) break;
+    am = an;
+    qm = qn;
+  }
+  m = lo;
+  const double left = line_diff(A(lo - 1), Q(lo - 1), am, qm, s, err);
+  const double right = line_diff(A(lo + 1), Q(lo + 1), am, qm, s, err);
+  return fmin(left, right) > gap + (double)err;
+}
+
+// Whether the ends of the ray are clear of the first and the last boundary.
+__device__ __forceinline__ bool list_ends_clear(const WalkRec* rec, int n, double len,
+                                                double gap) {
+  const WalkRec a = rec[0], b = rec[1], c = rec[n - 1], d = rec[n];
+  float e0 = 0.f, e1 = 0.f;
+  return line_diff(b.a, b.q, a.a, a.q, 0.0, e0) > gap + (double)e0 &&
+         line_diff(c.a, c.q, d.a, d.q, len, e1) > gap + (double)e1;
 }
 
 // Whether the reference's walk over the cells rec[0..n], whose boundaries are all
 // certified, inserts and accepts exactly them: every split point it visits has to
 // fall on one cell clear of its neighbours (see the head of this file).  `gap`
 // bounds the difference of squared distances that counts as clear, `room` the
-// pending points; `depth` receives the most there were.
+// pending points; `depth` receives the most there were.  (A form in which the
+// warp replays a ray's disjoint stretches together on a copy in shared memory
+// was slower: 32.1 against 30.8 ms on clustered_2m, 189 against 166 ms on
+// batched_1m; the 25 KB a block are missing from the L1 of the march.)
 __device__ __forceinline__ bool list_replay(const WalkRec* rec, int n, double gap, int room,
-                                            int& depth) {
+                                         int& depth) {
   int stack[kBatchStack];
   int i = 0, j = n, sp = 0;
-  double ai = rec[0].a, qi = rec[0].q, aj = rec[n].a, qj = rec[n].q;
   depth = 1;
   for (;;) {
     if (j == i + 1) {  // accepted
       if (sp == 0) return true;
       i = j;
-      ai = aj;
-      qi = qj;
       j = stack[--sp];
-      aj = rec[j].a;
-      qj = rec[j].q;
       continue;
     }
-    const double s = 0.5 * ((ai + aj) + (qj - qi) / (aj - ai));
-    const int m = list_find(rec, i + 1, j - 1, s);
-    const WalkRec r = rec[m];
-    if (!((double)r.slope * (s - r.t) > gap) ||
-        !((double)rec[m + 1].slope * (rec[m + 1].t - s) > gap) || sp + 1 >= room)
+    const double s = line_cross(rec[i].a, rec[i].q, rec[j].a, rec[j].q);
+    int m;
+    if (!list_nearest([&](int k) { return rec[k].a; }, [&](int k) { return rec[k].q; }, i, j, s,
+                      gap, m) ||
+        sp + 1 >= room)
       return false;
     stack[sp++] = j;
     depth = max(depth, sp + 1);
     j = m;
-    aj = r.a;
-    qj = r.q;
   }
 }
 
@@ -339,7 +382,9 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
   const int lane = threadIdx.x & 31;
   WalkRec* rec = io.rec + ((int64_t)blockIdx.x * kListBlock + threadIdx.x) * io.rec_cap;
   const Fetch64 f64{nullptr, c.nodes, 0};
-  unsigned n_rays = 0, n_cross = 0, n_q = 0, n_res = 0, max_sp = 0, n_visit = 0;
+  const Fetch32 f32{nullptr, c.nodes32, 0};
+  unsigned n_rays = 0, n_cross = 0, n_q = 0, n_res = 0, max_sp = 0;
+  unsigned n_visit = 0, n_ver = 0, n_qver = 0;  // (not reported by this kernel)
 
   for (;;) {
     // ---- the warp's next rays (neighbours in the coherent order)
@@ -352,6 +397,7 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
     bool live = lane < io.batch && slot < io.nrays;
     RayGeom g = {};
     double qm = 0.0;  // bounds the magnitude of all coordinates of the walk
+    double q_err = 0.0;  // FP32 error of its queries' coordinates
     if (live) {
       ray = io.order ? (int64_t)io.order[slot] : slot;
       ray_init(g, io.starts + 3 * ray, io.ends + 3 * ray);
@@ -364,7 +410,9 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
         for (int k = 0; k < 3; ++k) {
           qm = fmax(qm, fmax(fabs(g.s[k]), fabs(g.e[k])));
           qm = fmax(qm, fmax(fabs(c.bblo[k]), fabs(c.bbhi[k])));
+          q_err = fmax(q_err, fmax(fabs(g.s[k] - c.origin[k]), fabs(g.e[k] - c.origin[k])));
         }
+        q_err = q_err * 6.0e-8 + (double)c.coord_err;
       }
     }
 
@@ -381,7 +429,7 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
       while (__any_sync(FULL, phase < 4)) {
         const bool turn = phase < 4 && !on;
         bool query = turn;
-        double x = 0.0, y = 0.0, z = 0.0, R = pinf();
+        double x = 0.0, y = 0.0, z = 0.0, R = pinf(), dc = 0.0, dn = 0.0;
         if (turn && phase < 3) {
           x = phase == 1 ? g.s[0] : g.e[0];
           y = phase == 1 ? g.s[1] : g.e[1];
@@ -389,14 +437,24 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
         } else if (turn) {
           // the boundary point between the march's cell and its candidate; the
           // generators nearer than its two cells' distance plus the gap decide
-          const double4 pc = ldg_pt(&c.pts[cur]), pn = ldg_pt(&c.pts[m.nxt]);
-          double ac, qc, an, qn, off[3];
+          const double4 pc = ldg_pt(&c.pts[cur]);
+          double ac, qc, an, qn, tb, off[3];
           foot(g, pc, ac, qc, off);
-          foot(g, pn, an, qn, off);
-          const double tb = 0.5 * ((an + ac) + (qn - qc) / (an - ac));
-          if (an > ac && tb <= g.len) {
+          double4 pn;
+          bool in;
+          for (int k = 0;; ++k) {
+            pn = ldg_pt(&c.pts[m.nxt]);
+            foot(g, pn, an, qn, off);
+            tb = 0.5 * ((an + ac) + (qn - qc) / (an - ac));
+            in = an > ac && tb <= g.len;
+            if (in || k || m.nxt == m.c1) break;
+            m.nxt = m.c1;  // the list's best lies past the end: towards the last cell
+          }
+          if (in) {
             ray_point(g, tb, x, y, z);
-            R = fmax(metric(x, y, z, pc), metric(x, y, z, pn));
+            dc = metric(x, y, z, pc);
+            dn = metric(x, y, z, pn);
+            R = fmax(dc, dn);
             r_ask = 2.f * sqrtf((float)R);
             R += 4e-9 + 4e-14 * qm * (double)r_ask;
           } else {  // no such boundary: c1 ends the sequence, not certified
@@ -413,7 +471,10 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
         r.clear();
         if (query) {
           ++n_q;
-          knn64_fetch(c, f64, x, y, z, R, r, n_visit);
+          if (phase < 3) knn64_fetch(c, f64, x, y, z, R, r, n_visit);
+          else
+            knn3_guarded(c, f32, x, y, z, cur, m.nxt, dc, dn, R, guard_band(R, q_err), r, n_visit,
+                         n_ver, n_qver);
         }
         __syncwarp();
         if (query && r.id[0] < 0) {
@@ -441,8 +502,7 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
         } else if (query) {
           const double4 pc = ldg_pt(&c.pts[cur]), pn = ldg_pt(&c.pts[m.nxt]);
           const bool own = r.id[0] == cur || r.id[0] == m.nxt;
-          if (!own && r.r2[0] < fmin(metric(x, y, z, pc), metric(x, y, z, pn)) &&
-              ++m.tries < kListTries) {
+          if (!own && r.r2[0] < fmin(dc, dn) && ++m.tries < kListTries) {
             m.nxt = r.id[0];  // a nearer cell lies between
           } else {
             float w[3];
@@ -480,16 +540,15 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
     const bool one = live && m.c1 == c0;  // both ends in one cell
     const double gap = 4e-9 + 4e-14 * qm * (double)m.rho_max;
     bool whole = one;
-    if (live && !one) {
-      int depth = 0;
-      // boundaries close to the ray's ends are left to the walk below
-      const double edge = 1e-12 + 1e-13 * qm;
+    {
       const int room = io.local_cap < kBatchStack ? io.local_cap : kBatchStack;
-      whole = m.all && 2 * (int64_t)nrec <= io.max_iter && rec[1].t > edge &&
-              g.len - rec[nrec].t > edge && list_replay(rec, nrec, gap, room, depth);
+      const bool may = live && !one && m.all && 2 * (int64_t)nrec <= io.max_iter &&
+                       list_ends_clear(rec, nrec, g.len, gap);
+      int depth = 0;
+      if (may) whole = list_replay(rec, nrec, gap, room, depth);
+      __syncwarp();
       if (whole) max_sp = max(max_sp, (unsigned)depth);
     }
-    __syncwarp();
     std::conditional_t<OUT == kOutTape, TapeReducer<MODE, NF, true>, Reducer<MODE, NF>> red = {};
     FillSink fill = {};
     AdjSink<MODE, NF> adj = {};
@@ -610,15 +669,18 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
             dsub(nxt_s, cur_s) < 1e-14)
           return false;
         if (ni == ci + 1) {
-          if (!(rec[ni].slope > 0.f)) return false;
+          if (signbit(rec[ni].q)) return false;
           ++iter;
           accept();
           return live;
         }
-        const int k = list_find(rec, ci + 1, ni - 1, s);
-        const WalkRec a = rec[k], b = rec[k + 1];
-        if (a.cell == cur || a.cell == nxt || !((double)a.slope * (s - a.t) > gap) ||
-            !((double)b.slope * (b.t - s) > gap) || st.room() < 1)
+        int k;
+        if (!list_nearest([&](int e) { return rec[e].a; }, [&](int e) { return rec[e].q; }, ci, ni,
+                          s, gap, k))
+          return false;
+        const WalkRec a = rec[k];
+        if (a.cell == cur || a.cell == nxt || signbit(a.q) || signbit(rec[k + 1].q) ||
+            st.room() < 1)
           return false;
         ++iter;
         st_li[st.sp] = k;
@@ -720,10 +782,15 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
             fail(kNeedSlow);
           } else {
             // back on the list when the pushed cell is the recorded one
-            const int k0 = list_find(rec, 0, nrec, s);
+            int k0 = 0;
+            for (int hi = nrec; k0 < hi;) {  // the last foot up to s
+              const int mid = (k0 + hi + 1) >> 1;
+              if (rec[mid].a <= s) k0 = mid;
+              else hi = mid - 1;
+            }
             auto push = [&](int id) {
               int li = -1;
-              for (int k = max(k0 - 1, 0); k <= min(k0 + 1, nrec); ++k)
+              for (int k = max(k0 - 2, 0); k <= min(k0 + 2, nrec); ++k)
                 if (rec[k].cell == id) li = k;
               st_li[st.sp] = li;
               st.push(id, s);

@@ -524,15 +524,15 @@ static int sort_rays(vt_cloud* cl, WalkIO& io, cudaStream_t st) {
   return sort_rays_into(cl->view, io, cl->ws_order.p, total, cub_bytes, st);
 }
 
-// Four times the crossings of a ray through a homogeneous cloud; a longer ray
-// goes on with tree queries.
+// Six times the cube root of the cloud's size: four times the crossings of a ray
+// through a homogeneous cloud; a longer ray goes on with tree queries.
 int list_scratch(const vt_cloud* cl, int64_t nrays, int64_t& threads, int& cap) {
   int dev = 0, nsms = 0;
   VT_CUDA(cudaGetDevice(&dev));
   VT_CUDA(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev));
   threads = list_blocks(nrays, nsms) * kListBlock;
-  const int want = (int)(4.0 * std::cbrt((double)cl->npart)) & ~63;
-  cap = want < 256 ? 256 : (want > 2048 ? 2048 : want);
+  const int want = (int)(6.0 * std::cbrt((double)cl->npart)) & ~63;
+  cap = want < 256 ? 256 : (want > 4032 ? 4032 : want);
   return VT_OK;
 }
 

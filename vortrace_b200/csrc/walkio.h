@@ -36,14 +36,13 @@ constexpr int kErrNonFinite = 16;
 
 struct WalkDiag;
 
-// One cell of a marched ray (listed.cuh): the parameter t of the boundary into
-// it, the parameter a of its generator's foot on the ray, the foot's squared
-// distance q from the generator, and the rate at which the squared distances to
-// the boundary's two cells part along the ray (0: not certified).  One sector.
-struct __align__(32) WalkRec {
-  double t, a, q;
+// One cell of a marched ray (listed.cuh): the parameter a of its generator's foot
+// on the ray and the foot's squared distance q from the generator; the sign bit
+// of q is set when the boundary into the cell is not certified.
+struct __align__(16) WalkRec {
+  double a;
+  float q;
   int32_t cell;
-  float slope;
 };
 
 struct WalkIO {
