@@ -56,10 +56,11 @@ extern "C" {
 
 /* ---- walk kernels ------------------------------------------------------ */
 #define VT_KERNEL_AUTO 0        /* one ray per thread on neighbour lists built  */
-                                /* on first need; before that, on periodic      */
-                                /* clouds and on trees with leaves of more than */
-                                /* 8 points: THREAD_FP32, BATCHED below 65,536  */
-                                /* rays, or the autotuner's choice              */
+                                /* on first need; before that and on trees with */
+                                /* leaves of more than 8 points: THREAD_FP32,   */
+                                /* BATCHED below 65,536 rays, or the            */
+                                /* autotuner's choice.  Periodic clouds have one */
+                                /* kernel for every value but PLAIN_FP64        */
 #define VT_KERNEL_PLAIN_FP64 1  /* one ray per thread in the caller's order,    */
                                 /* full-FP64 k-NN from the root                 */
 #define VT_KERNEL_BATCHED 2     /* persistent queue, one warp per ray,          */

@@ -515,9 +515,9 @@ static __device__ __noinline__ RareOut rare_split(const DevCloud& c, RayGeom g, 
 }
 
 // Case 1a (src/ray.cpp:364-422): intermediate cells on both sides.
-static __device__ __noinline__ RareOut rare_case1a(const DevCloud& c, RayGeom g, double x, double y,
-                                            double z, int cur, int nxt) {
-  Search64 S(c);
+template <class Srch>
+__device__ __forceinline__ RareOut case1a(const RayGeom& g, Srch& S, double x, double y, double z,
+                                          int cur, int nxt) {
   int sc = try_along_ray(g, S, x, y, z, -1.0, cur, nxt);
   if (sc < 0) {
     const double ex = dmul(kPerturbEps, g.d[0]), ey = dmul(kPerturbEps, g.d[1]),
@@ -538,6 +538,11 @@ static __device__ __noinline__ RareOut rare_case1a(const DevCloud& c, RayGeom g,
                                                                   : 0;
   RareOut o{0.0, rc, sc, sn, S.nq};
   return o;
+}
+static __device__ __noinline__ RareOut rare_case1a(const DevCloud& c, RayGeom g, double x, double y,
+                                            double z, int cur, int nxt) {
+  Search64 S(c);
+  return case1a(g, S, x, y, z, cur, nxt);
 }
 
 // 100-NN classification (src/ray.cpp:319-338).

@@ -266,24 +266,37 @@ __device__ __noinline__ bool knn_tieorder(const DevCloud& c, double qx, double q
   return true;
 }
 
-// PointCloud::minDistSqToBox (src/pointcloud.cpp:283-297)
-__device__ __forceinline__ double min_dist_sq_to_box(const DevCloud& c, double x, double y,
-                                                     double z) {
-  const double q[3] = {x, y, z};
-  double d2 = 0.0;
+// PointCloud::minDistSqToBox (src/pointcloud.cpp:283-297) of the 27 periodic
+// images of a query, by axis: c[d][i + 1] is the squared distance that axis d adds
+// for the image shifted by i box sides, and the distance of an image is their sum in
+// axis order (an axis inside the domain adds nothing, and adding 0 is exact).
+struct ImageDist {
+  double c[3][3];
+  __device__ __forceinline__ ImageDist(const DevCloud& cl, double x, double y, double z) {
+    const double q[3] = {x, y, z};
 #pragma unroll
-  for (int dim = 0; dim < 3; dim++) {
-    const double lo = c.sub_lo[dim], hi = c.sub_hi[dim];
-    if (q[dim] < lo) {
-      const double d = dsub(lo, q[dim]);
-      d2 = dadd(d2, dmul(d, d));
-    } else if (q[dim] > hi) {
-      const double d = dsub(q[dim], hi);
-      d2 = dadd(d2, dmul(d, d));
+    for (int d = 0; d < 3; d++) {
+      const double lo = cl.sub_lo[d], hi = cl.sub_hi[d];
+#pragma unroll
+      for (int i = -1; i <= 1; i++) {
+        const double s = i ? dadd(q[d], dmul((double)i, cl.box[d])) : q[d];
+        const double g = s < lo ? dsub(lo, s) : (s > hi ? dsub(s, hi) : 0.0);
+        c[d][i + 1] = dmul(g, g);
+      }
     }
   }
-  return d2;
-}
+  __device__ __forceinline__ double operator()(int ix, int iy, int iz) const {
+    return dadd(dadd(c[0][ix + 1], c[1][iy + 1]), c[2][iz + 1]);
+  }
+  // no image but the query itself within `reach`: sums of non-negative terms
+  // round to at least each term, so one axis beyond it rules an image out
+  __device__ __forceinline__ bool none(double reach) const {
+    bool far = true;
+#pragma unroll
+    for (int d = 0; d < 3; d++) far = far && c[d][0] > reach && c[d][2] > reach;
+    return far;
+  }
+};
 
 // Periodic images of PointCloud::queryTreeK (src/pointcloud.cpp:308-368):
 // `res` holds the k-NN of q itself; each of the 26 shifted queries whose
@@ -296,9 +309,12 @@ template <int KMAX, bool TT, class L>
 __device__ __noinline__ void knn_periodic_merge64(const DevCloud& c, double qx, double qy,
                                                   double qz, L& res, unsigned& nvisit) {
   const int k = res.capacity();
+  int mn = res.count();
+  // most queries are farther from every face than from their k-th neighbour
+  const ImageDist dist(c, qx, qy, qz);
+  if (mn >= k && dist.none(dadd(res.worst(), kTol))) return;
   double md[2 * KMAX];
   int mi[2 * KMAX];
-  int mn = res.count();
   for (int i = 0; i < mn; i++) {
     md[i] = res.r2[i];
     mi[i] = res.id[i];
@@ -310,7 +326,7 @@ __device__ __noinline__ void knn_periodic_merge64(const DevCloud& c, double qx, 
         const double sx = dadd(qx, dmul((double)ix, c.box[0]));
         const double sy = dadd(qy, dmul((double)iy, c.box[1]));
         const double sz = dadd(qz, dmul((double)iz, c.box[2]));
-        const double minD2 = min_dist_sq_to_box(c, sx, sy, sz);
+        const double minD2 = dist(ix, iy, iz);
         const double worst = mn >= k ? md[k - 1] : __longlong_as_double(0x7ff0000000000000ULL);
         if (minD2 > dadd(worst, kTol)) continue;
         L img;
@@ -408,15 +424,16 @@ __device__ __forceinline__ int nn1_query(const DevCloud& c, double qx, double qy
   nn1_search<TT>(c, qx, qy, qz, id, d, tie, nvisit);
   if (id < 0) return -1;
   if constexpr (PER) {
-    if (c.periodic) {
+    const ImageDist dist(c, qx, qy, qz);
+    if (c.periodic && !dist.none(dadd(d, kTol))) {
       for (int ix = -1; ix <= 1; ix++)
         for (int iy = -1; iy <= 1; iy++)
           for (int iz = -1; iz <= 1; iz++) {
             if (ix == 0 && iy == 0 && iz == 0) continue;
+            if (dist(ix, iy, iz) > dadd(d, kTol)) continue;
             const double sx = dadd(qx, dmul((double)ix, c.box[0]));
             const double sy = dadd(qy, dmul((double)iy, c.box[1]));
             const double sz = dadd(qz, dmul((double)iz, c.box[2]));
-            if (min_dist_sq_to_box(c, sx, sy, sz) > dadd(d, kTol)) continue;
             int iid;
             double idd;
             nn1_search<TT>(c, sx, sy, sz, iid, idd, tie, nvisit);

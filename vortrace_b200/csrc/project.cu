@@ -115,12 +115,6 @@ static int launch_kind(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int ker
 // synchronisation, so the sequence can be captured into a CUDA graph.
 static int enqueue_walk(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel,
                         cudaStream_t st) {
-  // periodic clouds: the periodic k-NN merge and minimum-image split points
-  // live in the exact FP64 walk of the one-ray-per-thread kernel
-  if (cl->periodic) {
-    kernel = VT_KERNEL_PLAIN_FP64;
-    io.order = nullptr;
-  }
   io.max_iter = cl->max_iter;
   io.local_cap = cl->local_stack;
   io.cache_mode = cl->cache_mode;
@@ -549,7 +543,7 @@ int run_walk(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel, cudaS
     }
     io.rec = cl->ws_rec.p;
   }
-  if (kernel != VT_KERNEL_PLAIN_FP64 && !cl->periodic) {
+  if (kernel != VT_KERNEL_PLAIN_FP64) {
     const int rc = sort_rays(cl, io, st);
     if (rc) return rc;
   } else {
@@ -663,7 +657,7 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
       io.rec = g->rec.p;
     }
     size_t total = 0, cub_bytes = 0;
-    if (k != VT_KERNEL_PLAIN_FP64 && !cl->periodic) {
+    if (k != VT_KERNEL_PLAIN_FP64) {
       if ((rc = sort_rays_bytes(io.nrays, total, cub_bytes))) return rc;
       if (total && (rc = g->order.alloc(total))) return rc;
     }

@@ -390,8 +390,9 @@ __global__ void __launch_bounds__(128) k_slow(DevCloud c, WalkIO io) {
 // with warp-cooperative search (warp.cuh)
 #include "batched.cuh"
 #include "warp.cuh"
-// one ray per thread on the neighbour lists
+// one ray per thread on the neighbour lists; periodic clouds
 #include "listed.cuh"
+#include "periodic.cuh"
 
 namespace vt {
 
@@ -403,6 +404,9 @@ int launch_walk_t(vt_cloud* cl, WalkIO& io, int kernel, cudaStream_t st) {
     const int B = 128;
     if (io.deferred) {
       // second pass over the rays deferred for the reference-order tree
+    } else if (cl->periodic && kernel != VT_KERNEL_PLAIN_FP64) {
+      const int rc = launch_periodic<MODE, NF, OUT>(cl, io, st);
+      if (rc) return rc;
     } else if (cl->periodic) {
       k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
     } else if (kernel == kKernelList) {

@@ -7,8 +7,10 @@ B200.  Extras that do not change the reference's calls:
   * ``kernel`` attribute: ``'auto'`` (one ray per thread on neighbour
     lists, which are built when the cloud has seen enough rays to pay for
     them; before that the batched guarded-FP32 kernel, one ray per warp below
-    65,536 rays, or the autotuner's choice), ``'thread_fp32'``, ``'batched_fp64'``, ``'batched'`` (one ray per
-    warp), ``'plain'`` (one ray per thread in the caller's order, FP64);
+    65,536 rays, or the autotuner's choice), ``'thread_fp32'``,
+    ``'batched_fp64'``, ``'batched'`` (one ray per warp), ``'plain'`` (one ray
+    per thread in the caller's order, FP64).  Periodic clouds have one kernel
+    for all of these but ``'plain'``;
   * ``last_stats``: counters of the last projection (rays, crossings,
     queries, FP64 re-resolves, handed-over rays, walk time);
   * :meth:`batch_projection`: many grids and arbitrary rays in one launch;
