@@ -100,7 +100,7 @@ int vt::resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays) {
 }
 
 // The list walk (listed.cuh) takes every AUTO launch once the neighbour lists
-// are built, whatever the autotuner chose among the tree kernels (4.2 times
+// are built, whatever the autotuner chose among the tree kernels (4.9 times
 // faster at 1M rays, twice at 300).  Building them costs about 3 ns a point and
 // the allocation of 1 KB a point (2M points: 7 ms), a crossing on the tree 0.9 ns
 // (1M rays) to 6 ns (16,384 rays), so they are built when the crossings walked on
