@@ -202,6 +202,16 @@ int vt_knn(const vt_cloud *cloud, const double *q, uint64_t nq, int k, int64_t *
  * reloading the device tree drops it. */
 int vt_cloud_build_tie_tree(vt_cloud *cloud);
 
+/* The neighbour lists of the list walk, for diagnosis: 256 floats and one
+ * header word per point in tree order (the permutation of the saved tree),
+ * host buffers.  Group g of a point's 16 is {vx[4], vy[4], vz[4], tree index[4]}
+ * with v the vector to the neighbour; the vz > 0 part fills the groups 0, 1, ...,
+ * the other part 15, 14, ....  The header holds half the squared radius inside
+ * which the list is complete (FP32, low 10 bits cleared) and the parts' group
+ * counts (5 bits each, the vz > 0 part in the higher ones); 0: no list.
+ * VT_ERR_RUNTIME while the lists are not built. */
+int vt_cloud_neighbour_lists(vt_cloud *cloud, float *lists, uint32_t *headers);
+
 /* ---- projections ------------------------------------------------------- */
 /* Projection(starts, ends) + makeProjection(cloud, mode) + returnProjection
  * (src/projection.cpp:10-73, src/bindings.cpp:178-201).  Host buffers:

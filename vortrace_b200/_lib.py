@@ -50,7 +50,7 @@ EXPORTS = (
     "vt_tape_adjoint_device", "vt_slice", "vt_brute_projection", "vt_cloud_autotune",
     "vt_graph_create", "vt_graph_launch", "vt_graph_finish", "vt_graph_destroy",
     "vt_cloud_tree_save", "vt_cloud_tree_load", "vt_grid_rays_device", "vt_project_grid",
-    "vt_cloud_build_tie_tree", "vt_project_batch",
+    "vt_cloud_build_tie_tree", "vt_project_batch", "vt_cloud_neighbour_lists",
 )
 
 
@@ -151,6 +151,7 @@ def _open(p: str):
                                   C.POINTER(vp)]
     L.vt_cloud_build_tree.argtypes = [vp]
     L.vt_cloud_build_tie_tree.argtypes = [vp]
+    L.vt_cloud_neighbour_lists.argtypes = [vp, C.POINTER(C.c_float), C.POINTER(C.c_uint32)]
     L.vt_cloud_set_param.argtypes = [vp, C.c_int, C.c_int64]
     L.vt_cloud_set_fields.argtypes = [vp, dp]
     L.vt_cloud_set_fields_device.argtypes = [vp, vp, vp]
@@ -195,7 +196,7 @@ def _open(p: str):
                                          C.POINTER(Stats)]
     L.vt_tape_adjoint_device.argtypes = [vp, vp, vp, vp, u64, C.c_int, vp, vp, vp, vp]
     for name in ("vt_cloud_create", "vt_cloud_build_tree", "vt_cloud_build_tie_tree",
-                 "vt_cloud_set_param",
+                 "vt_cloud_neighbour_lists", "vt_cloud_set_param",
                  "vt_cloud_set_fields", "vt_cloud_set_fields_device",
                  "vt_cloud_get_info", "vt_cloud_orig_ids", "vt_knn", "vt_project",
                  "vt_project_device", "vt_project_device_noalloc", "vt_project_detailed",

@@ -329,6 +329,18 @@ int vt_cloud_tree_save(vt_cloud* cl, void* buf, uint64_t cap, uint64_t* size) {
   VT_GUARD_END
 }
 
+int vt_cloud_neighbour_lists(vt_cloud* cl, float* lists, uint32_t* headers) {
+  VT_GUARD_BEGIN
+  if (!cl || !lists || !headers) return set_error(VT_ERR_INVALID, "null argument");
+  std::lock_guard<std::mutex> lk(cl->mu);
+  if (!cl->view.nbr) return set_error(VT_ERR_RUNTIME, "the neighbour lists are not built");
+  VT_CUDA(cudaSetDevice(cl->device));
+  VT_CUDA(cudaMemcpy(lists, cl->view.nbr, cl->nbr_d.bytes(), cudaMemcpyDeviceToHost));
+  VT_CUDA(cudaMemcpy(headers, cl->view.nbr_hdr, cl->nbr_hdr_d.bytes(), cudaMemcpyDeviceToHost));
+  return VT_OK;
+  VT_GUARD_END
+}
+
 int vt_cloud_tree_load(vt_cloud* cl, const void* buf, uint64_t size) {
   VT_GUARD_BEGIN
   if (!cl || !buf) return set_error(VT_ERR_INVALID, "null argument");

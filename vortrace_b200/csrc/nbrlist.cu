@@ -19,8 +19,22 @@
 // One warp per leaf: it gathers the tree's points within a radius of the
 // leaf's box (the radius from the density of an ancestor of 32 to 63 points),
 // 32 nodes five levels down per step, keeps their coordinates relative to
-// the leaf in shared memory as FP32, and each of the leaf's points selects and
-// sorts its own (128-element bitonic sort, four elements per lane).
+// the leaf's first point in shared memory as FP32, and each of the leaf's points
+// selects its own from them and sorts them by their squared distance from the FP64
+// coordinates (128-element bitonic sort, four elements per lane).
+//
+// Why every point nearer than rho is listed.  u = 2^-24; S is the largest
+// gathered coordinate vector relative to the leaf's first point.  The FP32 vector
+// from the point to a gathered one differs from the true one by the rounding of
+// both (u S each at most) and of their difference (u d): its length is off by 2 u S
+// + 3 u d at most, sum of squares included, and the selection's radius re = ri + e
+// by 3 u re, so that e = 6 u (S + ri) lets all points at d <= ri in.  Of these,
+// 60 are kept in the order of the FP64 distance rounded to FP32 (u) without its 10
+// lowest bits (1.3e-4 of d^2), and rho is the first one left out, or ri, less
+// 1e-4 of rho^2 for the roundings.  A leaf can be as wide as the gaps between
+// compact groups, so that S / ri has no bound: with e in the place of a fixed
+// share of rho the radius stays true, and a point whose e is not small against
+// the distances selects too many and gets no list.
 #include "common.cuh"
 #include "internal.h"
 
@@ -174,6 +188,7 @@ __global__ void __launch_bounds__(kNbrWarps * 32)
   float r = cbrtf(ex * ey * ez * ((float)kNbrTarget / 4.18879f) / cnt);
   if (!(r > 0.02f * fmaxf(ex, fmaxf(ey, ez)))) r = 0.5f * fmaxf(ex, fmaxf(ey, ez));
   const double4 P0 = ldg_pt(&c.pts[a]);
+  float s_max = 0.f;  // largest gathered coordinate vector
   int m = -1;
   if (r > 0.f && r < 1e15f) {
     for (int t = 0; t < 12 && m < 0; ++t) {
@@ -181,31 +196,34 @@ __global__ void __launch_bounds__(kNbrWarps * 32)
       __syncwarp();
       if (m < 0) r *= 0.75f;
     }
+    for (int j = lane; j < m; j += 32)
+      s_max = fmaxf(s_max, S.x[j] * S.x[j] + S.y[j] * S.y[j] + S.z[j] * S.z[j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s_max = fmaxf(s_max, __shfl_xor_sync(kAll, s_max, o));
+    s_max = sqrtf(s_max);
   }
   for (int64_t i = a; i < b; ++i) {
     const double4 P = ldg_pt(&c.pts[i]);
     const float x = __double2float_rn(P.x - P0.x), y = __double2float_rn(P.y - P0.y),
                 z = __double2float_rn(P.z - P0.z);
-    // the points nearer than ri (at most kNbrKeys: a smaller ri when there are more)
+    // the points nearer than ri (at most kNbrKeys: a smaller ri when there are
+    // more), by their FP32 distance, which is off by less than e
     float ri2 = r * r;
     int k = 0;
     bool fits = false;
     for (int t = 0; t < 8 && m > 0 && !fits; ++t) {
       k = 0;
+      const float ri = sqrtf(ri2), re = ri + 3.6e-7f * (s_max + ri);
       for (int j0 = 0; j0 < m; j0 += 32) {
         const int j = j0 + lane;
-        float d2 = 0.f;
         bool in = false;
         if (j < m && S.id[j] != (int)i) {
           const float dx = S.x[j] - x, dy = S.y[j] - y, dz = S.z[j] - z;
-          d2 = dx * dx + dy * dy + dz * dz;
-          in = d2 <= ri2;
+          in = dx * dx + dy * dy + dz * dz <= re * re;
         }
         const unsigned im = __ballot_sync(kAll, in);
         const int at = k + __popc(im & ((1u << lane) - 1u));
-        // key: the squared distance with its 10 lowest mantissa bits replaced
-        // by the gathered slot
-        if (in && at < kNbrKeys) S.key[at] = (__float_as_uint(d2) & ~1023u) | (unsigned)j;
+        if (in && at < kNbrKeys) S.key[at] = (unsigned)j;
         k += __popc(im);
       }
       __syncwarp();
@@ -217,13 +235,22 @@ __global__ void __launch_bounds__(kNbrWarps * 32)
     if (fits && k > 0) {
       unsigned v[4];
 #pragma unroll
-      for (int h = 0; h < 4; ++h) v[h] = lane + 32 * h < k ? S.key[lane + 32 * h] : kAll;
+      for (int h = 0; h < 4; ++h) {
+        // key: the squared distance with its 10 lowest mantissa bits replaced
+        // by the gathered slot
+        v[h] = kAll;
+        if (lane + 32 * h < k) {
+          const unsigned j = S.key[lane + 32 * h];
+          const double4 Q = ldg_pt(&c.pts[S.id[j]]);
+          const double dx = dsub(Q.x, P.x), dy = dsub(Q.y, P.y), dz = dsub(Q.z, P.z);
+          v[h] = (__float_as_uint(__double2float_rn(dx * dx + dy * dy + dz * dz)) & ~1023u) | j;
+        }
+      }
       sort128(v, lane);
       const int kept = min(k, kNbrMax);
-      // complete up to the first point left out, or up to ri (rounding of the
-      // relative FP32 coordinates: 1e-5 at most, against 1e-4)
+      // complete up to the first point left out, or up to ri
       const unsigned next = __shfl_sync(kAll, v[kNbrMax >> 5], kNbrMax & 31);
-      const float rho2 = k > kNbrMax ? __uint_as_float(next & ~1023u) : ri2;
+      const float rho2 = k > kNbrMax ? fminf(__uint_as_float(next & ~1023u), ri2) : ri2;
       half_rho2 = 0.5f * rho2 * 0.9999f;
       // the two parts: ranks of this lane's points in theirs
       float vx[2], vy[2], vz[2];

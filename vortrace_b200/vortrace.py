@@ -105,6 +105,16 @@ class _Cloud:
     def set_param(self, param, value):
         L.check(self._lib.vt_cloud_set_param(self._h, param, int(value)))
 
+    def neighbour_lists(self):
+        """The list walk's lists (n, 16, 4, 4) and headers (n,), in tree order
+        (vt_cloud_neighbour_lists)."""
+        n = self.get_npart()
+        lists, head = np.empty((n, 16, 4, 4), np.float32), np.empty(n, np.uint32)
+        L.check(self._lib.vt_cloud_neighbour_lists(
+            self._h, lists.ctypes.data_as(C.POINTER(C.c_float)),
+            head.ctypes.data_as(C.POINTER(C.c_uint32))))
+        return lists, head
+
     # tree persistence (src/bindings.cpp:119-133)
     def saveTreeToBytes(self) -> bytes:
         size = C.c_uint64()
