@@ -93,7 +93,6 @@ int vt::check_projectable(const vt_cloud* cl, int mode) {
 // earlier: 16,384 rays of uniform_100k 174 / 188).
 // vt_cloud_autotune replaces the rule by its measured choice for batches of
 // at least its sample's size.
-constexpr uint64_t kThreadKernelMinRays = 65536;
 int vt::resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays) {
   if (cl->tuned_kernel != VT_KERNEL_AUTO && nrays >= cl->tuned_min_rays) return cl->tuned_kernel;
   return nrays < kThreadKernelMinRays ? VT_KERNEL_BATCHED : VT_KERNEL_THREAD_FP32;
@@ -109,7 +108,10 @@ int vt::resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays) {
 constexpr double kNbrCrossingsPerPoint = 1.0;
 int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
   if (kernel != VT_KERNEL_AUTO) return kernel == kKernelList ? VT_KERNEL_BATCHED_FP64 : kernel;
-  if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64) {
+  // (squares of distances above 1e16 do not leave FP32 much room)
+  double extent = 0.0;
+  for (int d = 0; d < 3; ++d) extent = fmax(extent, cl->view.bbhi[d] - cl->view.bblo[d]);
+  if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64 && extent <= 1e16) {
     cl->nbr_credit += 1.5 * std::cbrt((double)cl->npart) * (double)nrays;
     if (cl->nbr_credit >= kNbrCrossingsPerPoint * (double)cl->npart) {
       const int rc = build_nbr_lists(cl);

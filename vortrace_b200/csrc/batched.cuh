@@ -561,6 +561,7 @@ static __device__ __noinline__ RareOut rare_expand(const DevCloud& c, double x, 
 template <int MODE, int NF, int OUT, bool G32, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_batched(DevCloud c, WalkIO io, int nsm) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  if (launch_idle(io)) return;
   // stage the top tree levels
   if (G32) {
     // one pad entry in front, as in the global array: siblings share a
@@ -595,6 +596,7 @@ __global__ void __launch_bounds__(128, MINB) k_batched(DevCloud c, WalkIO io, in
   std::conditional_t<OUT == kOutTape, TapeReducer<MODE, NF, true>, Reducer<MODE, NF>> red;
   FillSink fill;
   AdjSink<MODE, NF> adj;
+  unsigned skip = 0;  // segments of the ray that an earlier launch emitted
   // lane counters
   unsigned n_rays = 0, n_cross = 0, n_q = 0, n_res = 0, n_visit = 0, n_ver = 0, max_sp = 0;
   unsigned n_qver = 0, n_q32 = 0;
@@ -618,12 +620,12 @@ __global__ void __launch_bounds__(128, MINB) k_batched(DevCloud c, WalkIO io, in
     if (need) {
       const int leader = __ffs(need) - 1;
       unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(&io.stats->next_ray, (unsigned long long)__popc(need));
+      if (lane == leader) base = atomicAdd(launch_queue(io), (unsigned long long)__popc(need));
       base = __shfl_sync(FULL, base, leader);
       if (want) {
         const int64_t i = (int64_t)base + __popc(need & ((1u << lane) - 1));
-        if (i < io.nrays) {
-          const int64_t r = io.order ? (int64_t)io.order[i] : i;
+        if (i < launch_rays(io)) {
+          const int64_t r = launch_ray(io, i, skip);
           ray = r;
           ray_init(g, io.starts + 3 * r, io.ends + 3 * r);
           if (!ray_finite(g)) {
@@ -633,9 +635,9 @@ __global__ void __launch_bounds__(128, MINB) k_batched(DevCloud c, WalkIO io, in
             ++n_rays;
             if (OUT == kOutImage || OUT == kOutCount || OUT == kOutTape)
               red.init(&c, io.out + r * io.nout);
-            if constexpr (OUT == kOutTape) red.set_tape(&io, r, 0u);
+            if constexpr (OUT == kOutTape) red.set_tape(&io, r, skip);
             else if (OUT == kOutFill) fill.init(&c, io, r);
-            else adj.init(&c, io, r, 0u);
+            else adj.init(&c, io, r, skip);
             double m = 0.0;
 #pragma unroll
             for (int j = 0; j < 3; ++j)
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(128, MINB) k_batched(DevCloud c, WalkIO io, in
       phase = 0;
     };
     auto fail = [&](int rc) {
-      if (rc == kNeedSlow || rc == kNeedTie) hand_over(io, ray, nseg_of());
+      if (rc == kNeedSlow || rc == kNeedTie) hand_over(io, ray, max(nseg_of(), skip));
       else report(io, ray, rc);
       max_sp = max(max_sp, (unsigned)st.maxsp);
       phase = 0;

@@ -172,6 +172,8 @@ struct DevStats {
   unsigned long long slow_count;   // rays queued for the degenerate kernel
   unsigned long long next_ray;     // work-queue head of the batched kernel
   unsigned long long next_slow;    // work-queue head of the degenerate kernel
+  unsigned long long redo_count;   // rays the list walk left to the tree kernels
+  unsigned long long next_redo;    // ... and the work-queue head over them
   unsigned long long search_steps;     // nodes (groups) the searches expanded
   unsigned long long fp64_checks;      // FP64 re-checks of FP32-passing points
   unsigned long long cache_refreshes;  // neighbourhood-cache refills (k_warp)

@@ -174,6 +174,9 @@ void drop_tie_tree(vt_cloud* cl);
 // fit) and free (the tree was rebuilt or reloaded)
 int build_nbr_lists(vt_cloud* cl);
 void drop_nbr_lists(vt_cloud* cl);
+// batches of at least this many rays run one ray per thread, smaller ones one
+// ray per warp (resolve_tree_kernel)
+constexpr uint64_t kThreadKernelMinRays = 65536;
 // the list walk (listed.cuh); chosen by resolve_kernel only
 constexpr int kKernelList = -1;
 // threads and boundaries per thread of its launch over nrays rays

@@ -18,7 +18,11 @@
 //           ray is reduced from it with the reference's FP64 split points;
 //   walk    for the other rays (0.1% on clustered_2m) the reference's own loop
 //           with FP64 queries on the tree, except where certified boundaries
-//           give the answer.
+//           give the answer.  A ray with many split points that the 3-NN does not
+//           decide, or with more than two queries per cell, is left to the tree
+//           kernels, launched next over what is left: clouds that the lists do not
+//           fit (lattices, cells near the tolerance) cost little more than without
+//           lists.
 //
 // The march is only a hint: results are the reference's bit for bit.  A boundary
 // is certified when every generator other than its two cells is farther from the
@@ -60,8 +64,14 @@ namespace vt {
 #define VT_LIST_WAIT 7
 #endif
 constexpr int kListBlock = 128;
-constexpr int kListRare = 16;
 constexpr int kListTries = 64;
+// a ray that needs more than kListAsks + 2 x cells tree queries is left to the
+// tree kernels
+constexpr int kListAsks = 64;
+// degenerate split points of a ray that are resolved here, and the most lanes of a
+// warp that may meet one together
+constexpr int kListRare = 4;
+constexpr int kListRareLanes = 2;
 
 __device__ __forceinline__ float rcp_approx(float x) {
   float y;
@@ -395,6 +405,7 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
     const int64_t slot = (int64_t)base + lane;
     int64_t ray = -1;
     bool live = lane < io.batch && slot < io.nrays;
+    int asks = 0;  // tree queries of this ray but for its ends'
     RayGeom g = {};
     double qm = 0.0;  // bounds the magnitude of all coordinates of the walk
     double q_err = 0.0;  // FP32 error of its queries' coordinates
@@ -415,6 +426,14 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
         q_err = q_err * 6.0e-8 + (double)c.coord_err;
       }
     }
+
+    // a ray that degenerate split points, overflow or too many queries keep from the
+    // list is walked again by the tree kernels, which skip what is emitted
+    auto give_up = [&](unsigned emitted) {
+      leave(io, ray, emitted);
+      --n_rays;
+      live = false;
+    };
 
     // ---- end cells and march.  A lane whose next step follows from its list
     // goes on; the others' queries run together once they are half of the
@@ -466,6 +485,12 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
             query = false;
           }
         }
+        // a ray that asks twice a cell is as well off on the tree
+        if (query && phase == 3 && ++asks > kListAsks + 2 * m.i) {
+          give_up(0u);
+          phase = 4;
+          query = false;
+        }
         __syncwarp();
         KnnList<3> r;
         r.clear();
@@ -478,7 +503,10 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
         }
         __syncwarp();
         if (query && r.id[0] < 0) {
-          report(io, ray, kErrNonFiniteDist);
+          // squared distances overflow: in FP64 an error, in the guarded FP32 of
+          // the march not yet one
+          if (phase < 3) report(io, ray, kErrNonFiniteDist);
+          else give_up(0u);
           live = false;
           phase = 4;
         } else if (query && phase < 3) {
@@ -637,15 +665,15 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
           finish_ok();
         }
       };
-      // The rare paths call functions that search for themselves: one lane at a
-      // time (an earlier form of this kernel, in which several lanes of a warp
-      // called a non-inlined search while the others waited at a warp barrier,
-      // never came back), and at most kListRare calls a ray, whose remainder is
-      // then left to k_slow.
+      // Degenerate split points (parallel bisectors, more than two cells at one
+      // distance) take the functions of the tree kernels, one lane at a time.  A few
+      // of the rays through a dense core meet one; where several lanes do, the cloud
+      // is a lattice or the like and the rays are left to the tree kernels.
       int rares = 0;
       auto one_by_one = [&](bool want, auto call) {
-        if (want && ++rares > kListRare) {
-          fail(kNeedSlow);
+        const int together = __popc(__ballot_sync(FULL, want));
+        if (want && (together > kListRareLanes || ++rares > kListRare)) {
+          give_up(nseg_of());
           want = false;
         }
         for (unsigned w = __ballot_sync(FULL, want); w; w &= w - 1) {
@@ -716,8 +744,9 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
             }
           } else {
             s = split_analytic(g, pc, pn);
-            query = true;
-            rare = !(s < DBL_MAX * 0.5 && s >= cur_s - kTol && s <= nxt_s + kTol);
+            query = ++asks <= kListAsks + 2 * nrec;
+            rare = query && !(s < DBL_MAX * 0.5 && s >= cur_s - kTol && s <= nxt_s + kTol);
+            if (!query) give_up(nseg_of());
           }
         }
         one_by_one(rare, [&] {  // parallel bisectors

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(kNbrWarps * 32)
   const float cnt = (float)(c.n >> (c.depth - up));
   const float4 al = __ldg(&c.boxlo[anc]), ah = __ldg(&c.boxhi[anc]);
   const float ex = ah.x - al.x, ey = ah.y - al.y, ez = ah.z - al.z;
-  float r = cbrtf(ex * ey * ez * ((float)kNbrTarget / 4.18879f) / cnt);
+  float r = cbrtf(ex) * cbrtf(ey) * cbrtf(ez) * cbrtf((float)kNbrTarget / 4.18879f / cnt);
   if (!(r > 0.02f * fmaxf(ex, fmaxf(ey, ez)))) r = 0.5f * fmaxf(ex, fmaxf(ey, ez));
   const double4 P0 = ldg_pt(&c.pts[a]);
   float s_max = 0.f;  // largest gathered coordinate vector

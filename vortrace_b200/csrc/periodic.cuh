@@ -19,6 +19,8 @@ namespace vt {
 #define VT_PERIODIC_MINB 4
 #endif
 
+constexpr int kPeriodicRare = 16;
+
 // 100-NN classification and Case 1a on a periodic cloud, not inlined
 static __device__ __noinline__ RareOut rare_expand_periodic(const DevCloud& c, double x, double y,
                                                             double z, int cur, int nxt) {
@@ -163,7 +165,7 @@ __global__ void __launch_bounds__(128, VT_PERIODIC_MINB) k_periodic(DevCloud c, 
     // the rare functions search for themselves: one lane at a time (see k_list)
     int rares = 0;
     auto one_by_one = [&](bool want, auto call) {
-      if (want && ++rares > kListRare) {
+      if (want && ++rares > kPeriodicRare) {
         fail(kNeedSlow);
         want = false;
       }

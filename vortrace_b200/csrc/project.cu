@@ -461,11 +461,13 @@ static int sort_rays_bytes(int64_t n, size_t& total, size_t& cub_bytes) {
 }
 
 // Enqueue the ray sort into `base` (sort_rays_bytes of scratch) and point
-// io.order at the result; no host synchronisation.
+// io.order at the result and io.redo_q at room for every ray; no host
+// synchronisation.
 static int sort_rays_into(const DevCloud& view, WalkIO& io, uint8_t* base, size_t total,
                           size_t cub_bytes, cudaStream_t st) {
   const int64_t n = io.nrays;
   io.order = nullptr;
+  io.redo_q = nullptr;
   if (total == 0) return VT_OK;
   SortLayout L;
   int rc = sort_rays_layout(n, L);
@@ -488,6 +490,7 @@ static int sort_rays_into(const DevCloud& view, WalkIO& io, uint8_t* base, size_
   VT_CUDA(cudaGetLastError());
   size_t cb = L.cub_rays;
   VT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, cb, k0, k1, i0, i1, (int)n, 0, 63, st));
+  io.redo_q = k0;  // the unsorted keys are read no more: 8 bytes a ray
   int dev = 0, nsms = 0;
   VT_CUDA(cudaGetDevice(&dev));
   VT_CUDA(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev));

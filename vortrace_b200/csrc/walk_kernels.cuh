@@ -11,6 +11,7 @@
 // stack), k_batched (batched.cuh) and k_warp (warp.cuh).
 #pragma once
 
+#include <climits>
 #include <type_traits>
 
 #include "internal.h"
@@ -317,6 +318,35 @@ __device__ __forceinline__ void hand_over(const WalkIO& io, int64_t ray, unsigne
   io.slow_q[k] = ((unsigned long long)ray << 24) | (emitted & 0xffffffu);
 }
 
+// The same for the tree kernels, which walk the ray again from its start after the
+// list walk.
+__device__ __forceinline__ void leave(const WalkIO& io, int64_t ray, unsigned emitted) {
+  const unsigned long long k = atomicAdd(&io.stats->redo_count, 1ULL);
+  io.redo_q[k] = ((unsigned long long)ray << 24) | (emitted & 0xffffffu);
+}
+// Rays of a tree kernel's launch, the head of their queue, and its i-th ray with
+// the segments that the list walk emitted for it.
+__device__ __forceinline__ int64_t launch_rays(const WalkIO& io) {
+  return io.redo ? (int64_t)io.stats->redo_count : io.nrays;
+}
+__device__ __forceinline__ bool launch_idle(const WalkIO& io) {
+  if (!io.redo) return false;
+  const long long n = launch_rays(io);
+  return n < io.redo_lo || n >= io.redo_hi;
+}
+__device__ __forceinline__ unsigned long long* launch_queue(const WalkIO& io) {
+  return io.redo ? &io.stats->next_redo : &io.stats->next_ray;
+}
+__device__ __forceinline__ int64_t launch_ray(const WalkIO& io, int64_t i, unsigned& skip) {
+  skip = 0u;
+  if (io.redo) {
+    const unsigned long long e = io.redo_q[i];
+    skip = (unsigned)(e & 0xffffffu);
+    return (int64_t)(e >> 24);
+  }
+  return io.order ? (int64_t)io.order[i] : i;
+}
+
 // ------------------------------------------------------------ k_plain
 template <int MODE, int NF, int OUT, bool PER>
 __global__ void __launch_bounds__(128) k_plain(DevCloud c, WalkIO io) {
@@ -410,7 +440,23 @@ int launch_walk_t(vt_cloud* cl, WalkIO& io, int kernel, cudaStream_t st) {
     } else if (cl->periodic) {
       k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
     } else if (kernel == kKernelList) {
-      const int rc = launch_list<MODE, NF, OUT>(cl, io, st);
+      // the list walk, then the tree kernels over the rays it left, whose number is
+      // not known here: one warp per ray takes few of them, one thread per ray many
+      // (a launch that finds no rays of its own takes 2 us)
+      int rc = launch_list<MODE, NF, OUT>(cl, io, st);
+      if (rc) return rc;
+      VT_CUDA(cudaGetLastError());
+      const bool warps = cl->nfields <= 32;
+      io.redo = 1;
+      io.redo_lo = 1;
+      io.redo_hi = warps ? (long long)kThreadKernelMinRays : LLONG_MAX;
+      if (warps) rc = launch_warp<MODE, OUT>(cl, io, st);
+      if (!rc && (!warps || io.nrays >= (int64_t)kThreadKernelMinRays)) {
+        if (warps) io.redo_lo = (long long)kThreadKernelMinRays;
+        io.redo_hi = LLONG_MAX;
+        rc = launch_batched<MODE, NF, OUT>(cl, io, VT_KERNEL_THREAD_FP32, st);
+      }
+      io.redo = 0;
       if (rc) return rc;
     } else if (kernel == VT_KERNEL_PLAIN_FP64) {
       k_plain<MODE, NF, OUT, false><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);

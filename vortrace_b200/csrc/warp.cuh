@@ -662,6 +662,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
   __shared__ float4 cache_all[kWarpsPerBlock][kCache];
   __shared__ float4 cblo_all[kWarpsPerBlock][kChunks];
   __shared__ float4 cbhi_all[kWarpsPerBlock][kChunks];
+  if (launch_idle(io)) return;
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;
   int* s_node = s_node_all[wib];
@@ -682,10 +683,11 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
 
   for (;;) {
     long long ray = 0;
-    if (lane == 0) ray = (long long)atomicAdd(&io.stats->next_ray, 1ULL);
+    if (lane == 0) ray = (long long)atomicAdd(launch_queue(io), 1ULL);
     ray = __shfl_sync(kFull, ray, 0);
-    if (ray >= io.nrays) break;
-    if (io.order) ray = io.order[ray];
+    if (ray >= launch_rays(io)) break;
+    unsigned skip;  // segments of the ray that an earlier launch emitted
+    ray = launch_ray(io, ray, skip);
     RayGeom g;
     ray_init(g, io.starts + 3 * ray, io.ends + 3 * ray);
     if (!ray_finite(g)) {
@@ -697,6 +699,10 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
 #pragma unroll
     for (int j = 0; j < 3; ++j)
       qe = fmax(qe, fmax(fabs(g.s[j] - c.origin[j]), fabs(g.e[j] - c.origin[j])));
+    if (qe > 1e18 || cerr > 6e10) {  // squares that leave FP32
+      if (lane == 0) hand_over(io, ray, skip);
+      continue;
+    }
     qe = qe * 6.0e-8 + cerr;
 
     WarpReducer<MODE> red;
@@ -705,7 +711,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
     int64_t fill_off = 0;
     if (OUT == kOutImage || OUT == kOutCount || OUT == kOutTape) red.init();
     else if (OUT == kOutFill) fill_off = io.offsets[ray];
-    else adj.init(io, lane, ray, 0u);
+    else adj.init(io, lane, ray, skip);
     auto emit = [&](int cell, double a, double b) {
       if (OUT == kOutImage || OUT == kOutCount) red.seg(c, lane, cell, a, b);
       else if (OUT == kOutTape) {
@@ -717,8 +723,9 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
           const double p0 = __shfl_sync(kFull, red.acc, 0);
           const double p1 = __shfl_sync(kFull, red.acc, 1);
           const double p2 = __shfl_sync(kFull, red.acc, 2);
-          if (lane == 0) tape_append(io, TapeEntryV{cell, (int)ray, dsub(b, a), T0, {p0, p1, p2}});
-        } else if (lane == 0) {
+          if (lane == 0 && red.nseg > skip)
+            tape_append(io, TapeEntryV{cell, (int)ray, dsub(b, a), T0, {p0, p1, p2}});
+        } else if (lane == 0 && red.nseg > skip) {
           tape_append(io, TapeEntry{c.perm[cell], (int)ray, dsub(b, a)});
         }
       } else if (OUT == kOutFill) {
@@ -780,7 +787,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
     const int c0 = nn_end(g.s[0], g.s[1], g.s[2]);
     const int c1 = nn_end(g.e[0], g.e[1], g.e[2]);
     if (c0 == kTieUnresolved || c1 == kTieUnresolved) {
-      if (lane == 0) hand_over(io, ray, 0u);
+      if (lane == 0) hand_over(io, ray, skip);
       continue;
     }
     if (c0 < 0 || c1 < 0) {
@@ -983,7 +990,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32, VT_WARP_MINB) k_warp(DevC
       }
       n_cross += nseg_now();
     } else if (lane == 0) {
-      if (rc == kNeedSlow || rc == kNeedTie) hand_over(io, ray, nseg_now());
+      if (rc == kNeedSlow || rc == kNeedTie) hand_over(io, ray, max(nseg_now(), skip));
       else report(io, ray, rc);
     }
     __syncwarp();
