@@ -19,7 +19,11 @@ namespace vt {
 #define VT_PERIODIC_MINB 4
 #endif
 
-constexpr int kPeriodicRare = 16;
+// degenerate split points of a ray that are resolved here, and the most lanes of a
+// warp that may meet one together (k_plain's own time is that of its longest ray, so
+// that a few rays are better kept)
+constexpr int kPeriodicRare = 64;
+constexpr int kPeriodicRareLanes = 8;
 
 // 100-NN classification and Case 1a on a periodic cloud, not inlined
 static __device__ __noinline__ RareOut rare_expand_periodic(const DevCloud& c, double x, double y,
@@ -162,11 +166,18 @@ __global__ void __launch_bounds__(128, VT_PERIODIC_MINB) k_periodic(DevCloud c, 
       else report(io, ray, rc);
       phase = kIdle;
     };
-    // the rare functions search for themselves: one lane at a time (see k_list)
+    // the rare functions search for themselves, one lane at a time; where several lanes
+    // want one together (a lattice) or a ray wants many, the rays are walked again by
+    // k_plain (30,000 rays along the columns of a 32^3 lattice: 24.6 ms one lane at a
+    // time, 7.6 by k_plain alone).  A caller without scratch for the queue
+    // (vt_project_device_noalloc) has them done here.
     int rares = 0;
     auto one_by_one = [&](bool want, auto call) {
-      if (want && ++rares > kPeriodicRare) {
-        fail(kNeedSlow);
+      const int together = __popc(__ballot_sync(FULL, want));
+      if (want && io.redo_q && (together > kPeriodicRareLanes || ++rares > kPeriodicRare)) {
+        leave(io, ray, nseg_of());
+        --n_rays;
+        phase = kIdle;
         want = false;
       }
       for (unsigned w = __ballot_sync(FULL, want); w; w &= w - 1) {

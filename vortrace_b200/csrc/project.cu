@@ -551,6 +551,7 @@ int run_walk(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel, cudaS
     if (rc) return rc;
   } else {
     io.order = nullptr;  // the plain kernel keeps the caller's order
+    io.redo_q = nullptr;
   }
   const int slow_threads = 1024;
   if (cl->ws_stats.reserve(1)) return VT_ERR_NOMEM;

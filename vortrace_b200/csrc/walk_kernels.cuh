@@ -318,14 +318,14 @@ __device__ __forceinline__ void hand_over(const WalkIO& io, int64_t ray, unsigne
   io.slow_q[k] = ((unsigned long long)ray << 24) | (emitted & 0xffffffu);
 }
 
-// The same for the tree kernels, which walk the ray again from its start after the
-// list walk.
+// The same for a kernel that walks the ray again from its start after the list walk
+// (the tree kernels) or the periodic one (k_plain).
 __device__ __forceinline__ void leave(const WalkIO& io, int64_t ray, unsigned emitted) {
   const unsigned long long k = atomicAdd(&io.stats->redo_count, 1ULL);
   io.redo_q[k] = ((unsigned long long)ray << 24) | (emitted & 0xffffffu);
 }
-// Rays of a tree kernel's launch, the head of their queue, and its i-th ray with
-// the segments that the list walk emitted for it.
+// Rays of such a kernel's launch, the head of their queue, and its i-th ray with the
+// segments that the first walk emitted for it.
 __device__ __forceinline__ int64_t launch_rays(const WalkIO& io) {
   return io.redo ? (int64_t)io.stats->redo_count : io.nrays;
 }
@@ -350,15 +350,17 @@ __device__ __forceinline__ int64_t launch_ray(const WalkIO& io, int64_t i, unsig
 // ------------------------------------------------------------ k_plain
 template <int MODE, int NF, int OUT, bool PER>
 __global__ void __launch_bounds__(128) k_plain(DevCloud c, WalkIO io) {
-  const int64_t ray = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (ray >= io.nrays) return;
+  const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (i >= launch_rays(io)) return;
+  unsigned skip;
+  const int64_t ray = launch_ray(io, i, skip);
   Search64T<PER> S(c);
   LocalStack<kPlainStack> st;
   st.set_cap(io.local_cap);
   st.clear();
   unsigned nseg = 0;
-  int rc = run_ray<MODE, NF, OUT>(c, io, ray, S, st, 0u, nseg);
-  if (rc == kNeedSlow || rc == kNeedTie) hand_over(io, ray, nseg);
+  int rc = run_ray<MODE, NF, OUT>(c, io, ray, S, st, skip, nseg);
+  if (rc == kNeedSlow || rc == kNeedTie) hand_over(io, ray, max(nseg, skip));
   report(io, ray, rc);
   warp_add(&io.stats->rays, 1u);
   warp_add(&io.stats->crossings, rc == 0 ? nseg : 0u);
@@ -437,6 +439,11 @@ int launch_walk_t(vt_cloud* cl, WalkIO& io, int kernel, cudaStream_t st) {
     } else if (cl->periodic && kernel != VT_KERNEL_PLAIN_FP64) {
       const int rc = launch_periodic<MODE, NF, OUT>(cl, io, st);
       if (rc) return rc;
+      if (io.redo_q) {  // the rays it left
+        io.redo = 1;
+        k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
+        io.redo = 0;
+      }
     } else if (cl->periodic) {
       k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
     } else if (kernel == kKernelList) {

@@ -75,9 +75,10 @@ struct WalkIO {
   WalkRec* rec;          // list walk: rec_cap boundaries per thread (NULL: not this kernel)
   int rec_cap;
   int batch;             // list walk: rays a warp takes at a time (1..32)
-  // rays that the list walk leaves to the tree kernels, as in slow_q, and for
-  // those kernels: walk these rays instead of 0..nrays-1, when there are at least
-  // redo_lo and fewer than redo_hi of them
+  // rays that the list walk leaves to the tree kernels, and the periodic one to
+  // k_plain, as in slow_q (NULL: none may be left), and for those kernels: walk these
+  // rays instead of 0..nrays-1 (tree kernels: when there are at least redo_lo and
+  // fewer than redo_hi of them)
   unsigned long long* redo_q;
   int redo;
   long long redo_lo, redo_hi;
