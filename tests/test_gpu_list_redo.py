@@ -2,7 +2,7 @@
 point on every ray), cells near the tolerance, a box of 1e16, against the
 one-ray-per-thread FP64 walk bit for bit (gradients within the rounding of their
 sums).  Ray counts on both sides of the switch between one ray per warp and one per
-thread; more than 32 fields."""
+thread, with 1 to 32 rays to a warp of the list walk; more than 32 fields."""
 import warnings
 
 import numpy as np
@@ -14,10 +14,13 @@ pytestmark = pytest.mark.gpu
 def _case(kind, nf):
     import vortrace_b200 as vt
     rng = np.random.default_rng(len(kind))
-    box = {"lattice": 16.0, "tiny": 2e-3, "huge": 1e16}[kind]
-    if kind == "lattice":
+    box = {"lattice": 16.0, "mixed": 16.0, "tiny": 2e-3, "huge": 1e16}[kind]
+    if kind in ("lattice", "mixed"):
         c = np.arange(16) + 0.5
         pos = np.stack(np.meshgrid(c, c, c, indexing="ij"), -1).reshape(-1, 3)
+        if kind == "mixed":  # random points in one half: both kinds of ray in a warp
+            move = pos[:, 0] > 8
+            pos[move] = rng.uniform(0, 16, (move.sum(), 3)) * [0.5, 1, 1] + [8, 0, 0]
     else:
         pos = rng.uniform(0, box, (4000, 3))
     f = rng.uniform(0, 1, (len(pos), nf))
@@ -40,7 +43,7 @@ def _with(pc, kernel, call):
     return call()
 
 
-@pytest.mark.parametrize("kind", ["lattice", "tiny", "huge"])
+@pytest.mark.parametrize("kind", ["lattice", "mixed", "tiny", "huge"])
 @pytest.mark.parametrize("m,nf,reduction", [(700, 1, "integrate"), (700, 2, "max"),
                                             (700, 33, "integrate"), (140001, 4, "volume"),
                                             (110001, 1, "integrate")])
@@ -72,7 +75,7 @@ def test_coordinates_whose_squares_leave_fp32(m):
         np.testing.assert_array_equal(pc.projection(s, e), want)
 
 
-@pytest.mark.parametrize("kind", ["lattice", "tiny"])
+@pytest.mark.parametrize("kind", ["lattice", "mixed", "tiny"])
 @pytest.mark.parametrize("m", [700, 110001])
 def test_segments_and_gradients(kind, m):
     import torch

@@ -31,13 +31,30 @@
 //   * generators outside the list are farther than rho >= 2 r + slack from
 //     the cell, r the boundary point's distance to it;
 //   * listed ones ahead of the ray: their bisector is crossed later than the
-//     chosen one by more than both error bounds (FP32 error 64 2^-24 rho^2 of
-//     half the difference of squared distances; the derivation needs 40);
-//   * listed ones behind the ray have receded since the entry point, so they
-//     are as far as the certified entry made them; only the cell the ray came
-//     from has to be looked at again.  Without a certified entry all listed
-//     ones are tested at the exit point;
+//     chosen one by more than both error bounds (below);
+//   * those behind the ray have receded since the entry point, so they are as far
+//     as the certified entry made them; only the cell the ray came from has to
+//     be looked at again.  Without a certified entry all listed ones are tested
+//     at the exit point;
 //   * or a bounded FP64 query at the boundary point finds its two cells only.
+// The FP32 error of half the difference of squared distances to cell P and a
+// listed point at v, num - tau den, in units of u = 2^-24 and with R = rho, |v| <= R,
+// entry |w| <= 2 R (tested), tau <= 2.5 R:
+//   entry point w     the rounding of d, of the entry before and of the steps from
+//                     there, R' the rho of the cell before: (6 R' + 4 R) R;
+//   num               v and v^2: 4.5 R^2, three fused steps of up to 2.5 R^2 and
+//                     the subtraction of thr: 10 R^2;
+//   tau               the approximate reciprocal and a product: 3 tau den: 7.5 R^2;
+//   den               d, v and three fused steps: 5 R.  6 R are added, so that a den
+//                     that is not positive is truly not: tau times 11 R: 27.5 R^2.
+// 53.5 R^2 + 6 R' R in all; thr is 64 R^2 + 6 R' R above 2e-9 and the FP64 term.  The
+// sign of den is what the points behind rest on: a ray that follows a face at an
+// angle of 1e-8 stays for the whole face within 1e-7 of both cells, far above the
+// tolerance, and a cell taken for behind that is not would be missed.
+// A point that is not listed keeps 1.25 thr at the computed exit, which is off by up
+// to thr / den: one that is crossed slower than the chosen point loses less than
+// thr there, and one crossed faster would put the next step's exit before its
+// entry, which is not certified.
 // At a split point s between certified boundaries t_m < s < t_(m+1) the
 // difference to every cell is a linear function that is above the bound at
 // both ends, except for the two neighbours in the sequence, whose difference is
@@ -104,6 +121,7 @@ struct March {
   float wx, wy, wz;    // entry point relative to the current cell's generator
   float px, py, pz;    // the same of `prev`, as it was used
   float den;           // rate of the entry boundary (half differences)
+  float rho_in;        // rho of the cell that the entry point was found from (0: FP64)
   float rho_chain;     // smallest rho since the points behind were last tested
   float rho_max;
   bool all;            // every settled boundary is certified
@@ -167,18 +185,22 @@ __device__ __forceinline__ int list_step(const DevCloud& c, const RayGeom& g, do
   }
   const float hrho = __uint_as_float(hdr & ~1023u);  // rho^2 / 2
   const float rho = sqrtf(2.f * hrho);
-  const float thr = 2e-9f + (float)(2e-14 * qm) * rho + 7.7e-6f * hrho;
+  const float thr =
+      2e-9f + fmaf((float)(2e-14 * qm) + 3.6e-7f * m.rho_in, rho, 7.7e-6f * hrho);
   const float w2 = fmaf(m.wx, m.wx, fmaf(m.wy, m.wy, m.wz * m.wz));
   const float wd = fmaf(m.wx, dx, fmaf(m.wy, dy, m.wz * dz));
   const float kInf = __int_as_float(0x7f800000);
   // candidate n: half the difference of squared distances at ray parameter tau
-  // past the entry is num - tau den (positive while the ray is nearer to cur);
+  // past the entry is num - tau den (positive while the ray is nearer to cur; den
+  // rounded up);
   // lo = (num - thr) / den bounds its exit from below, lo + 2 thr / den from
   // above.  The smallest lo with its group slot and 1 / den, and the next one.
   float lo1 = kInf, lo2 = kInf, inv1 = 0.f, r2 = kInf;
   int bi = -1;
   bool ended = false;
-  const float2 half2 = make_float2(0.5f, 0.5f), mthr2 = make_float2(-thr, -thr);
+  const float eps = 3.6e-7f * rho;
+  const float2 half2 = make_float2(0.5f, 0.5f), mthr2 = make_float2(-thr, -thr),
+               eps2 = make_float2(eps, eps);
   const float2 wx2 = make_float2(-m.wx, -m.wx), wy2 = make_float2(-m.wy, -m.wy),
                wz2 = make_float2(-m.wz, -m.wz);
   const float2 dx2 = make_float2(dx, dx), dy2 = make_float2(dy, dy), dz2 = make_float2(dz, dz);
@@ -218,7 +240,7 @@ __device__ __forceinline__ int list_step(const DevCloud& c, const RayGeom& g, do
             wx2, vx[p], __ffma2_rn(wy2, vy[p], __ffma2_rn(wz2, vz[p],
                                                           __ffma2_rn(half2, vv[p], mthr2))));
         const float2 den =
-            __ffma2_rn(dx2, vx[p], __ffma2_rn(dy2, vy[p], __fmul2_rn(dz2, vz[p])));
+            __ffma2_rn(dx2, vx[p], __ffma2_rn(dy2, vy[p], __ffma2_rn(dz2, vz[p], eps2)));
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           const float dj = j ? den.y : den.x;
@@ -278,6 +300,7 @@ __device__ __forceinline__ int list_step(const DevCloud& c, const RayGeom& g, do
   if (!ok) return kMarchAsk;
   m.rho_chain = chained ? fminf(m.rho_chain, rho) : rho;
   m.rho_max = fmaxf(m.rho_max, rho);
+  m.rho_in = rho;
   m.prev = cur;
   m.prev_clean = m.clean;
   m.px = m.wx;
@@ -538,6 +561,7 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
             m.prev = -1;
             m.clean = own && (r.id[1] == cur || r.id[1] == m.nxt) && r.id[2] < 0;
             m.rho_chain = r_ask;
+            m.rho_in = 0.f;
             m.rho_max = fmaxf(m.rho_max, r_ask);
             m.wx = (float)(x - pn.x);
             m.wy = (float)(y - pn.y);
