@@ -102,3 +102,32 @@ def test_segments_and_gradients(kind, m):
         L.dptr(np.ascontiguousarray(up.cpu().numpy())), L.dptr(grad)))
     np.testing.assert_allclose(grad, want.cpu().numpy(), rtol=1e-11,
                                atol=1e-13 * float(want.abs().max()))
+
+
+def test_ray_that_goes_round():
+    """A ray near a vertex of the mesh at large coordinates, on which the reference's
+    walk goes round within its tolerance until its iteration limit: the same error
+    from every kernel, also once the reference-order tree is there."""
+    import vortrace_b200 as vt
+    from vortrace_b200 import _lib as L
+    rng = np.random.default_rng(0)
+    pos = 1e4 * rng.uniform(0, 1, (rng.integers(70, 3000), 3)) + 1e5
+    s = np.array([[106511.39264565839, 103293.52250029893, 108495.26246356587]])
+    e = np.array([[106497.31696201646, 103146.07777772452, 108775.09324459988]])
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        pc = vt.ProjectionCloud(pos, np.ones(len(pos)), boundbox=[1e5, 1.1e5] * 3)
+    a, b = 1e5 + 1e4 * rng.uniform(0.1, 0.9, (2, 4000, 3))
+    pc.projection(a, b)
+    pc._cloud.neighbour_lists()  # they are built
+    want = pc.projection(a, b)
+    pc._cloud.set_param(L.PARAM_MAX_ITERATIONS, 2000)
+    for _ in range(2):
+        for kernel in ("plain", "auto", "batched"):
+            pc.kernel = kernel
+            with pytest.raises(L.VortraceError, match="maximum iteration count"):
+                pc.projection(s, e)
+            with pytest.raises(L.VortraceError, match="maximum iteration count"):
+                pc.traced_projection(s, e)
+    pc.kernel = "auto"
+    np.testing.assert_array_equal(pc.projection(a, b), want)

@@ -427,16 +427,20 @@ __global__ void k_permute_batches(const int32_t* __restrict__ order,
 
 // Scratch of the ray sort for n rays: keys and indices (twice), the batch
 // costs, keys and indices (twice) and CUB's temporary storage of both
-// sorts; 0 when the rays keep their order (few or too many).
+// sorts; when the rays keep their order (few or too many), only the first keys'
+// place, which io.redo_q takes in either case.
 struct SortLayout {
   size_t kb, ib, nbb, cub_rays, cub_batches, total;
+  bool sorted;
 };
 
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 static int sort_rays_layout(int64_t n, SortLayout& L) {
   L = SortLayout{};
-  if (n < 64 || n > (int64_t)0x7fffffff) return VT_OK;
+  L.total = L.kb = up256((size_t)n * 8);
+  L.sorted = n >= 64 && n <= (int64_t)0x7fffffff;
+  if (!L.sorted) return VT_OK;
   const int64_t nb = (n + kBatch - 1) / kBatch;
   VT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, L.cub_rays, (unsigned long long*)nullptr,
                                           (unsigned long long*)nullptr, (int32_t*)nullptr,
@@ -444,7 +448,6 @@ static int sort_rays_layout(int64_t n, SortLayout& L) {
   VT_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, L.cub_batches, (uint32_t*)nullptr,
                                           (uint32_t*)nullptr, (int32_t*)nullptr,
                                           (int32_t*)nullptr, (int)nb, 0, 32));
-  L.kb = up256((size_t)n * 8);
   L.ib = up256((size_t)n * 4);
   L.nbb = up256((size_t)nb * 4);
   // keys x2 | idx x2 | cost | batch keys x2 | batch idx x2 | cub (max of both)
@@ -468,11 +471,14 @@ static int sort_rays_into(const DevCloud& view, WalkIO& io, uint8_t* base, size_
   const int64_t n = io.nrays;
   io.order = nullptr;
   io.redo_q = nullptr;
-  if (total == 0) return VT_OK;
+  if (total == 0) return VT_OK;  // (graphs of the plain kernel)
   SortLayout L;
   int rc = sort_rays_layout(n, L);
   if (rc) return rc;
   if (L.total > total) return set_error(VT_ERR_RUNTIME, "ray sort scratch too small");
+  // the keys' place is free once they are sorted: 8 bytes a ray
+  io.redo_q = reinterpret_cast<unsigned long long*>(base);
+  if (!L.sorted) return VT_OK;
   const int64_t nb = (n + kBatch - 1) / kBatch;
   auto* k0 = reinterpret_cast<unsigned long long*>(base);
   auto* k1 = reinterpret_cast<unsigned long long*>(base + L.kb);
@@ -490,7 +496,6 @@ static int sort_rays_into(const DevCloud& view, WalkIO& io, uint8_t* base, size_
   VT_CUDA(cudaGetLastError());
   size_t cb = L.cub_rays;
   VT_CUDA(cub::DeviceRadixSort::SortPairs(tmp, cb, k0, k1, i0, i1, (int)n, 0, 63, st));
-  io.redo_q = k0;  // the unsorted keys are read no more: 8 bytes a ray
   int dev = 0, nsms = 0;
   VT_CUDA(cudaGetDevice(&dev));
   VT_CUDA(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev));
