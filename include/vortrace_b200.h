@@ -91,6 +91,15 @@ extern "C" {
 #define VT_PARAM_TUNE_LEAF_SIZE 11  /* 1: vt_cloud_autotune also times leaf    */
                                     /* sizes 6 and 12 (rebuilding the tree;    */
                                     /* default 0)                              */
+#define VT_PARAM_LIST_BYTES 12      /* most device memory in bytes that AUTO's */
+                                    /* neighbour lists (1,028 per point) and a */
+                                    /* launch's walk records (up to 2.3 GB at  */
+                                    /* 16M points; each graph has its own) may */
+                                    /* take; 0: none, AUTO stays on the tree;  */
+                                    /* default -1: a quarter of what is free   */
+                                    /* when they are built.  A value below     */
+                                    /* what built lists take frees them, and   */
+                                    /* graphs captured on them refuse to launch */
 
 typedef struct vt_cloud vt_cloud;
 typedef struct vt_segments vt_segments;
@@ -108,7 +117,8 @@ typedef struct {
   int32_t tree_depth;  /* internal levels of the implicit tree              */
   uint64_t tree_leaves;
   double tree_build_ms;
-  uint64_t device_bytes; /* device memory held by the handle                */
+  uint64_t device_bytes; /* device memory of the cloud, its trees and lists  */
+                         /* (without the workspaces of calls)                */
   uint64_t tie_tree_nodes; /* reference-order tree: nodes (0: not built)    */
   int32_t tie_tree_depth;  /* ... its depth in nodes                        */
   int32_t reserved;
@@ -333,9 +343,10 @@ int vt_cloud_tree_load(vt_cloud *cloud, const void *buf, uint64_t size);
  * captured once; vt_graph_launch replays them on `stream` with one
  * cudaGraphLaunch, reading the rays the buffers hold at that time.
  * vt_graph_finish waits for `stream`, returns the counters and reports a
- * failed ray like vt_project_device.  The graph owns its scratch; rebuilding
- * the cloud's tree or reallocating its fields invalidates it (launch then
- * fails).  Launches of one graph must not overlap. */
+ * failed ray like vt_project_device.  The graph owns its scratch.  It holds the
+ * addresses of the cloud's tree, fields and, captured on them, neighbour lists:
+ * after any rebuild, reload or reallocation of these, in place or not, launch
+ * fails.  Launches of one graph must not overlap. */
 int vt_graph_create(vt_cloud *cloud, const double *d_starts, const double *d_ends,
                     uint64_t nrays, int mode, int kernel, double *d_out, vt_graph **out);
 int vt_graph_launch(vt_graph *graph, void *stream);

@@ -36,6 +36,7 @@ PARAM_CACHE = 8
 PARAM_ADJOINT_KERNEL = 9
 PARAM_DETAILED_KERNEL = 10
 PARAM_TUNE_LEAF_SIZE = 11
+PARAM_LIST_BYTES = 12
 
 # every symbol the header declares (checked by the tests)
 EXPORTS = (

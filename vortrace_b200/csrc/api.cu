@@ -111,11 +111,15 @@ int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
   // (squares of distances above 1e16 do not leave FP32 much room)
   double extent = 0.0;
   for (int d = 0; d < 3; ++d) extent = fmax(extent, cl->view.bbhi[d] - cl->view.bblo[d]);
-  if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64 && extent <= 1e16) {
+  if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64 && extent <= 1e16 &&
+      cl->list_bytes != 0) {
     cl->nbr_credit += 1.5 * std::cbrt((double)cl->npart) * (double)nrays;
     if (cl->nbr_credit >= kNbrCrossingsPerPoint * (double)cl->npart) {
-      const int rc = build_nbr_lists(cl);
+      WalkIO io{};
+      io.nrays = (int64_t)nrays;
+      const int rc = build_nbr_lists(cl, list_scratch(cl, io) * sizeof(WalkRec));
       if (rc) return resolve_tree_kernel(cl, nrays);
+      if (!cl->view.nbr) cl->nbr_credit = 0.0;  // no room: not at every call
     }
   }
   return cl->view.nbr ? kKernelList : resolve_tree_kernel(cl, nrays);
@@ -412,6 +416,16 @@ int vt_cloud_set_param(vt_cloud* cl, int param, int64_t value) {
     case VT_PARAM_TUNE_LEAF_SIZE:
       if (value < 0 || value > 1) return set_error(VT_ERR_INVALID, "tune leaf size must be 0 or 1");
       cl->tune_leaf = (int)value;
+      return VT_OK;
+    case VT_PARAM_LIST_BYTES:
+      if (value < -1) return set_error(VT_ERR_INVALID, "list bytes must be >= -1");
+      cl->list_bytes = value;
+      if (cl->view.nbr && value >= 0 && (uint64_t)value < vt::nbr_list_bytes(cl)) {
+        VT_CUDA(cudaSetDevice(cl->device));
+        VT_CUDA(cudaDeviceSynchronize());  // no walk on another stream reads them
+        vt::drop_nbr_lists(cl);
+        cl->ws_rec.reset();
+      }
       return VT_OK;
     default:
       return set_error(VT_ERR_INVALID, "unknown parameter " + std::to_string(param));

@@ -124,6 +124,8 @@ struct vt_cloud {
   vt::DevBuf<float4> nbr_d;     // neighbour lists (nbrlist.cu) ...
   vt::DevBuf<uint32_t> nbr_hdr_d;
   double nbr_credit = 0.0;      // ... and the crossings walked without them
+  int64_t list_bytes = -1;      // most bytes they and a launch's records may take
+  uint64_t list_gen = 0;        // bumped when they are freed
   // reference-order tree (tietree.cu), built when an exact tie needs it
   vt::DevBuf<vt::TieNode> tt_nodes_d;
   vt::DevBuf<double4> tt_pts_d;
@@ -170,17 +172,18 @@ int build_tree_device(vt_cloud* cl);
 // and free (the device tree was rebuilt or reloaded)
 int build_tie_tree(vt_cloud* cl, cudaStream_t st);
 void drop_tie_tree(vt_cloud* cl);
-// neighbour lists (nbrlist.cu): build (no-op when built or when they do not
-// fit) and free (the tree was rebuilt or reloaded)
-int build_nbr_lists(vt_cloud* cl);
+// neighbour lists (nbrlist.cu): their bytes, build (no-op when built or when they
+// and `records` more do not fit) and free (the tree was rebuilt or reloaded)
+size_t nbr_list_bytes(const vt_cloud* cl);
+int build_nbr_lists(vt_cloud* cl, size_t records);
 void drop_nbr_lists(vt_cloud* cl);
 // batches of at least this many rays run one ray per thread, smaller ones one
 // ray per warp (resolve_tree_kernel)
 constexpr uint64_t kThreadKernelMinRays = 65536;
 // the list walk (listed.cuh); chosen by resolve_kernel only
 constexpr int kKernelList = -1;
-// threads and boundaries per thread of its launch over nrays rays
-int list_scratch(const vt_cloud* cl, int64_t nrays, int64_t& threads, int& cap);
+// io.batch and io.rec_cap of its launch over io.nrays rays; returns the records
+size_t list_scratch(const vt_cloud* cl, WalkIO& io);
 // saved trees (tree_build.cu)
 uint64_t tree_blob_size(const vt_cloud* cl);
 int save_tree_blob(vt_cloud* cl, void* buf);

@@ -413,7 +413,9 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
   constexpr bool kImage = OUT == kOutImage || OUT == kOutCount || OUT == kOutTape;
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  WalkRec* rec = io.rec + ((int64_t)blockIdx.x * kListBlock + threadIdx.x) * io.rec_cap;
+  // (lanes past io.batch have no ray and no records)
+  const int64_t warp = (int64_t)blockIdx.x * (kListBlock / 32) + (threadIdx.x >> 5);
+  WalkRec* rec = io.rec + (warp * io.batch + lane) * io.rec_cap;
   const Fetch64 f64{nullptr, c.nodes, 0};
   const Fetch32 f32{nullptr, c.nodes32, 0};
   unsigned n_rays = 0, n_cross = 0, n_q = 0, n_res = 0, max_sp = 0;
@@ -865,11 +867,17 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
   warp_max(&io.stats->max_stack, max_sp);
 }
 
-// Blocks of a launch over nrays rays on nsms SMs.
+// Blocks of a launch over nrays rays on nsms SMs, and the rays that a warp takes at
+// a time: few rays are spread over all resident warps.
 inline int64_t list_blocks(int64_t nrays, int nsms) {
   const int64_t blocks = (int64_t)nsms * VT_LIST_MINB;
   const int64_t need = (nrays + kListBlock / 32 - 1) / (kListBlock / 32);
   return need < blocks ? (need > 0 ? need : 1) : blocks;
+}
+inline int list_batch(int64_t nrays, int nsms) {
+  const int64_t warps = list_blocks(nrays, nsms) * (kListBlock / 32);
+  const int64_t per = (nrays + warps - 1) / warps;
+  return (int)(per < 32 ? (per < 1 ? 1 : per) : 32);
 }
 
 template <int MODE, int NF, int OUT>
@@ -878,9 +886,6 @@ int launch_list(vt_cloud* cl, WalkIO& io, cudaStream_t st) {
   VT_CUDA(cudaGetDevice(&dev));
   VT_CUDA(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t blocks = list_blocks(io.nrays, nsms);
-  const int64_t warps = blocks * (kListBlock / 32);
-  const int64_t per = (io.nrays + warps - 1) / warps;
-  io.batch = (int)(per < 32 ? (per < 1 ? 1 : per) : 32);
   k_list<MODE, NF, OUT><<<(unsigned)blocks, kListBlock, 0, st>>>(cl->view, io);
   return VT_OK;
 }

@@ -305,16 +305,27 @@ void drop_nbr_lists(vt_cloud* cl) {
   cl->nbr_hdr_d.reset();
   cl->view.nbr = nullptr;
   cl->view.nbr_hdr = nullptr;
+  ++cl->list_gen;
+}
+
+size_t nbr_list_bytes(const vt_cloud* cl) {
+  return (size_t)cl->npart * (kNbrGroups * 4 * sizeof(float4) + sizeof(uint32_t));
 }
 
 // Build the lists of a built, non-periodic cloud (no-op when built).  Without
-// the memory for them the cloud simply has none.
-int build_nbr_lists(vt_cloud* cl) {
+// the memory for them and for `records` bytes of walk records the cloud simply has
+// none.
+int build_nbr_lists(vt_cloud* cl, size_t records) {
   if (cl->view.nbr) return VT_OK;
   const size_t n = (size_t)cl->npart, count = n * kNbrGroups * 4;
-  size_t avail = 0, total = 0;
-  VT_CUDA(cudaMemGetInfo(&avail, &total));
-  if (count * sizeof(float4) + n * sizeof(uint32_t) > avail / 2) return VT_OK;
+  size_t most = (size_t)cl->list_bytes;
+  if (cl->list_bytes < 0) {
+    // a quarter of the free memory: a caller that shares the device keeps the rest
+    size_t total = 0;
+    VT_CUDA(cudaMemGetInfo(&most, &total));
+    most /= 4;
+  }
+  if (nbr_list_bytes(cl) + records > most) return VT_OK;
   if (cl->nbr_d.alloc(count) || cl->nbr_hdr_d.alloc(n)) {
     cudaGetLastError();  // not enough memory after all
     drop_nbr_lists(cl);

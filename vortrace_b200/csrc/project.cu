@@ -528,24 +528,22 @@ static int sort_rays(vt_cloud* cl, WalkIO& io, cudaStream_t st) {
 
 // Six times the cube root of the cloud's size: four times the crossings of a ray
 // through a homogeneous cloud; a longer ray goes on with tree queries.
-int list_scratch(const vt_cloud* cl, int64_t nrays, int64_t& threads, int& cap) {
+size_t list_scratch(const vt_cloud* cl, WalkIO& io) {
   int dev = 0, nsms = 0;
-  VT_CUDA(cudaGetDevice(&dev));
-  VT_CUDA(cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev));
-  threads = list_blocks(nrays, nsms) * kListBlock;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    nsms = 148;
   const int want = (int)(6.0 * std::cbrt((double)cl->npart)) & ~63;
-  cap = want < 256 ? 256 : (want > 4032 ? 4032 : want);
-  return VT_OK;
+  io.rec_cap = want < 256 ? 256 : (want > 4032 ? 4032 : want);
+  io.batch = list_batch(io.nrays, nsms);
+  return (size_t)(list_blocks(io.nrays, nsms) * (kListBlock / 32)) * io.batch * io.rec_cap;
 }
 
 // Walk launch with the handle's (grow-only) workspace as scratch.
 int run_walk(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel, cudaStream_t st,
              vt_stats* stats) {
   if (kernel == kKernelList) {
-    int64_t threads = 0;
-    const int rc = list_scratch(cl, io.nrays, threads, io.rec_cap);
-    if (rc) return rc;
-    if (cl->ws_rec.reserve((size_t)threads * io.rec_cap)) {
+    if (cl->ws_rec.reserve(list_scratch(cl, io))) {
       cudaGetLastError();  // no memory for the boundaries: walk on the tree
       kernel = resolve_tree_kernel(cl, io.nrays);
     }
@@ -611,7 +609,9 @@ struct vt_graph {
   vt::DevBuf<vt::WalkRec> rec;
   vt::WalkIO io{};
   int mode = 0;
-  uint64_t tree_gen = 0;  // the cloud's tree (and lists) at capture time
+  uint64_t tree_gen = 0;  // the cloud's tree at capture time
+  bool lists = false;     // captured on its lists ...
+  uint64_t list_gen = 0;  // ... of this generation
   const double4* pts = nullptr;  // the cloud's buffers at capture time
   const double* fields = nullptr;
   ~vt_graph() {
@@ -657,9 +657,7 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
     io.slow_threads = slow_threads;
     int k = resolve_kernel(cl, kernel, nrays);
     if (k == kKernelList) {
-      int64_t threads = 0;
-      if ((rc = list_scratch(cl, io.nrays, threads, io.rec_cap))) return rc;
-      if (g->rec.alloc((size_t)threads * io.rec_cap)) {
+      if (g->rec.alloc(list_scratch(cl, io))) {
         cudaGetLastError();
         k = resolve_tree_kernel(cl, nrays);
       }
@@ -690,6 +688,8 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
     g->graph = graph;
     VT_CUDA(cudaGraphInstantiate(&g->exec, graph, 0));
     g->tree_gen = cl->tree_gen;
+    g->lists = k == kKernelList;
+    g->list_gen = cl->list_gen;
     g->pts = cl->view.pts;
     g->fields = cl->view.fields;
     *out = g.release();
@@ -703,7 +703,7 @@ int vt_graph_launch(vt_graph* g, void* stream) {
   using namespace vt;
   if (!g) return set_error(VT_ERR_INVALID, "null graph handle");
   if (g->cl->view.pts != g->pts || g->cl->view.fields != g->fields ||
-      g->cl->tree_gen != g->tree_gen)
+      g->cl->tree_gen != g->tree_gen || (g->lists && g->cl->list_gen != g->list_gen))
     return set_error(VT_ERR_RUNTIME,
                      "the cloud's tree or fields were reallocated after the graph was created");
   VT_CUDA(cudaSetDevice(g->device));

@@ -72,7 +72,7 @@ struct WalkIO {
   void* tape;            // kOutTape: entries [0, tape_cap) (TapeEntry, or TapeEntryV for volume)
   unsigned long long* tape_count;  // kOutTape: entries appended (may exceed tape_cap)
   unsigned long long tape_cap;
-  WalkRec* rec;          // list walk: rec_cap boundaries per thread (NULL: not this kernel)
+  WalkRec* rec;          // list walk: rec_cap records for each of the rays in flight
   int rec_cap;
   int batch;             // list walk: rays a warp takes at a time (1..32)
   // rays that the list walk leaves to the tree kernels, and the periodic one to

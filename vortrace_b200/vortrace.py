@@ -474,6 +474,14 @@ class ProjectionCloud:
         ids, r2 = self._cloud.knn(q, k)
         return np.where(ids >= 0, self.orig_ids[np.maximum(ids, 0)], -1), r2
 
+    def limit_lists(self, nbytes: int) -> None:
+        """Let the neighbour lists of the ``'auto'`` kernel (1,028 bytes a cell) and
+        a call's walk records take at most ``nbytes`` of device memory (extension).
+        0: no lists, ``'auto'`` stays on the tree; -1 (the default): a quarter of
+        the memory that is free when they are built.  Lists that are larger are
+        freed."""
+        self._cloud.set_param(L.PARAM_LIST_BYTES, nbytes)
+
     def autotune(self, pos_start, pos_end, *, reduction="integrate",
                  max_sample: int = 1048576, leaf_size: bool = False) -> dict:
         """Time the walk kernels (rays per warp), shared-memory tree depths and
