@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   // (lanes past io.batch have no ray and no records)
-  const int64_t warp = (int64_t)blockIdx.x * (kListBlock / 32) + (threadIdx.x >> 5);
+  const unsigned warp = blockIdx.x * (kListBlock / 32) + (threadIdx.x >> 5);
   WalkRec* rec = io.rec + (warp * io.batch + lane) * io.rec_cap;
   const Fetch64 f64{nullptr, c.nodes, 0};
   const Fetch32 f32{nullptr, c.nodes32, 0};

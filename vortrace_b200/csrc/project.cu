@@ -157,6 +157,18 @@ static int complete_deferred(vt_cloud* cl, WalkIO& io, int out_kind, int mode, c
   return VT_OK;
 }
 
+// Rays that the first walk left (see `leave`), and the ones handed over from there.
+static int complete_redo(vt_cloud* cl, WalkIO& io, int out_kind, int mode, const DevStats& hs,
+                         cudaStream_t st) {
+  io.redo = 1;
+  io.redo_lo = (long long)hs.redo_count;
+  io.slow_from = hs.slow_count;
+  const int rc = launch_kind(cl, io, out_kind, mode, VT_KERNEL_AUTO, st);
+  io.redo = 0;
+  io.slow_from = 0;
+  return rc;
+}
+
 static int run_walk_on(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel,
                        cudaStream_t st, vt_stats* stats, WalkDiag* d_diag, bool timed,
                        bool may_alloc = true) {
@@ -166,7 +178,16 @@ static int run_walk_on(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int ker
     VT_CUDA(cudaEventCreate(&e1));
     VT_CUDA(cudaEventRecord(e0, st));
   }
-  const int rc = enqueue_walk(cl, io, out_kind, mode, kernel, st);
+  io.redo_late = 1;
+  int rc = enqueue_walk(cl, io, out_kind, mode, kernel, st);
+  DevStats hs;
+  for (int pass = 0; !rc && pass < 2; ++pass) {
+    if (timed) VT_CUDA(cudaEventRecord(e1, st));
+    VT_CUDA(cudaMemcpyAsync(&hs, io.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
+    VT_CUDA(cudaStreamSynchronize(st));
+    if (pass || hs.redo_count == 0) break;
+    rc = complete_redo(cl, io, out_kind, mode, hs, st);
+  }
   if (rc) {
     if (timed) {
       cudaEventDestroy(e0);
@@ -174,10 +195,6 @@ static int run_walk_on(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int ker
     }
     return rc;
   }
-  if (timed) VT_CUDA(cudaEventRecord(e1, st));
-  DevStats hs;
-  VT_CUDA(cudaMemcpyAsync(&hs, io.stats, sizeof(DevStats), cudaMemcpyDeviceToHost, st));
-  VT_CUDA(cudaStreamSynchronize(st));
   float ms = 0.f;
   if (timed) {
     cudaEventElapsedTime(&ms, e0, e1);

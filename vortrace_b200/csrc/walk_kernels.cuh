@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(128) k_slow(DevCloud c, WalkIO io) {
   st.cap = io.gstack_cap;
   st.clear();
   const unsigned long long total = io.stats->slow_count;
-  for (unsigned long long q = tid; q < total; q += io.slow_threads) {
+  for (unsigned long long q = io.slow_from + tid; q < total; q += io.slow_threads) {
     const unsigned long long e = io.slow_q[q];
     if (io.deferred && !(e & kDeferredBit)) continue;
     const int64_t ray = queued_ray(e);
@@ -429,6 +429,35 @@ __global__ void __launch_bounds__(128) k_slow(DevCloud c, WalkIO io) {
 namespace vt {
 
 // ------------------------------------------------------------ dispatch
+// The launch over the `n` rays that the list walk or the periodic one left (see
+// `leave`): one warp per ray for few of them, one thread per ray for many.  n < 0: not
+// known (a graph), a launch of either kind, of which one finds no rays of its own.
+template <int MODE, int NF, int OUT>
+int launch_redo(vt_cloud* cl, WalkIO& io, long long n, cudaStream_t st) {
+  constexpr long long few = (long long)kThreadKernelMinRays;
+  const bool warps = cl->nfields <= 32;
+  int rc = VT_OK;
+  io.redo = 1;
+  io.redo_lo = 1;
+  io.redo_hi = LLONG_MAX;
+  if (cl->periodic) {
+    const long long most = n < 0 ? io.nrays : n;
+    k_plain<MODE, NF, OUT, true><<<(unsigned)((most + 127) / 128), 128, 0, st>>>(cl->view, io);
+  } else {
+    if (warps && n < few) {
+      io.redo_hi = few;
+      rc = launch_warp<MODE, OUT>(cl, io, st);
+    }
+    if (!rc && (!warps || n >= few || (n < 0 && io.nrays >= few))) {
+      io.redo_lo = warps ? few : 1;
+      io.redo_hi = LLONG_MAX;
+      rc = launch_batched<MODE, NF, OUT>(cl, io, VT_KERNEL_THREAD_FP32, st);
+    }
+  }
+  io.redo = 0;
+  return rc;
+}
+
 template <int MODE, int NF, int OUT>
 int launch_walk_t(vt_cloud* cl, WalkIO& io, int kernel, cudaStream_t st) {
   const DevCloud& c = cl->view;
@@ -436,35 +465,20 @@ int launch_walk_t(vt_cloud* cl, WalkIO& io, int kernel, cudaStream_t st) {
     const int B = 128;
     if (io.deferred) {
       // second pass over the rays deferred for the reference-order tree
-    } else if (cl->periodic && kernel != VT_KERNEL_PLAIN_FP64) {
-      const int rc = launch_periodic<MODE, NF, OUT>(cl, io, st);
+    } else if (io.redo) {
+      // (io.redo_lo: the number of rays)
+      const int rc = launch_redo<MODE, NF, OUT>(cl, io, io.redo_lo, st);
       if (rc) return rc;
-      if (io.redo_q) {  // the rays it left
-        io.redo = 1;
-        k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
-        io.redo = 0;
+    } else if ((cl->periodic && kernel != VT_KERNEL_PLAIN_FP64) || kernel == kKernelList) {
+      int rc = cl->periodic ? launch_periodic<MODE, NF, OUT>(cl, io, st)
+                            : launch_list<MODE, NF, OUT>(cl, io, st);
+      if (!rc && !io.redo_late && io.redo_q) {
+        VT_CUDA(cudaGetLastError());
+        rc = launch_redo<MODE, NF, OUT>(cl, io, -1, st);
       }
+      if (rc) return rc;
     } else if (cl->periodic) {
       k_plain<MODE, NF, OUT, true><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
-    } else if (kernel == kKernelList) {
-      // the list walk, then the tree kernels over the rays it left, whose number is
-      // not known here: one warp per ray takes few of them, one thread per ray many
-      // (a launch that finds no rays of its own takes 2 us)
-      int rc = launch_list<MODE, NF, OUT>(cl, io, st);
-      if (rc) return rc;
-      VT_CUDA(cudaGetLastError());
-      const bool warps = cl->nfields <= 32;
-      io.redo = 1;
-      io.redo_lo = 1;
-      io.redo_hi = warps ? (long long)kThreadKernelMinRays : LLONG_MAX;
-      if (warps) rc = launch_warp<MODE, OUT>(cl, io, st);
-      if (!rc && (!warps || io.nrays >= (int64_t)kThreadKernelMinRays)) {
-        if (warps) io.redo_lo = (long long)kThreadKernelMinRays;
-        io.redo_hi = LLONG_MAX;
-        rc = launch_batched<MODE, NF, OUT>(cl, io, VT_KERNEL_THREAD_FP32, st);
-      }
-      io.redo = 0;
-      if (rc) return rc;
     } else if (kernel == VT_KERNEL_PLAIN_FP64) {
       k_plain<MODE, NF, OUT, false><<<(unsigned)((io.nrays + B - 1) / B), B, 0, st>>>(c, io);
     } else if (kernel == VT_KERNEL_BATCHED && cl->nfields <= 32) {

@@ -76,12 +76,14 @@ struct WalkIO {
   int rec_cap;
   int batch;             // list walk: rays a warp takes at a time (1..32)
   // rays that the list walk leaves to the tree kernels, and the periodic one to
-  // k_plain, as in slow_q (NULL: none may be left), and for those kernels: walk these
-  // rays instead of 0..nrays-1 (tree kernels: when there are at least redo_lo and
-  // fewer than redo_hi of them)
+  // k_plain, as in slow_q (NULL: none may be left)
   unsigned long long* redo_q;
+  // launch over those rays instead of 0..nrays-1, when there are at least redo_lo
+  // and fewer than redo_hi of them
   int redo;
   long long redo_lo, redo_hi;
+  int redo_late;  // the host launches it when it has seen their number
+  unsigned long long slow_from;  // k_slow: first entry of slow_q not yet finished
   WalkDiag* diag;
   int deferred;          // k_slow only, over the entries deferred for the
                          // reference-order tree (which is now built)
