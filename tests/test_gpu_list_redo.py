@@ -84,6 +84,7 @@ def test_segments_and_gradients(kind, m):
     pc, rng, box = _case(kind, 3)
     s, e = _rays(rng, m, box)
     pc.projection(s, e)
+    pc._cloud.buildTree()  # (the lists' next walks; AUTO may prefer the tree later)
     a, b = (_with(pc, k, lambda: pc.traced_projection(s, e, return_midpoint=False, flatten=True))
             for k in ("plain", "auto"))
     pc._cloud.neighbour_lists()
@@ -93,10 +94,12 @@ def test_segments_and_gradients(kind, m):
     up = torch.as_tensor(rng.normal(size=(m, 3)), device="cuda")
     want, = torch.autograd.grad(VA.project(pc, f, s, e, kernel="plain"), f, up)
     for _ in range(2):  # from the tape
+        pc._cloud.buildTree()
         got, = torch.autograd.grad(VA.project(pc, f, s, e), f, up)
         torch.testing.assert_close(got, want, rtol=1e-11, atol=1e-13 * float(want.abs().max()))
     grad = np.zeros((len(pc.orig_ids), 3))  # walked again
     out = np.ascontiguousarray(pc.projection(s, e))
+    pc._cloud.buildTree()
     L.check(pc._cloud._lib.vt_project_adjoint(
         pc._cloud._h, L.dptr(s), L.dptr(e), m, L.REDUCE_SUM, L.dptr(out),
         L.dptr(np.ascontiguousarray(up.cpu().numpy())), L.dptr(grad)))

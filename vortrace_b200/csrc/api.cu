@@ -55,6 +55,9 @@ bool verbose() { return g_verbose.load(); }
 
 using vt::check_projectable;
 using vt::resolve_kernel;
+using vt::WalkIO;
+using vt::WalkRec;
+using vt::DevStats;
 using vt::set_error;
 
 #define VT_GUARD_BEGIN try {
@@ -98,23 +101,63 @@ int vt::resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays) {
   return nrays < kThreadKernelMinRays ? VT_KERNEL_BATCHED : VT_KERNEL_THREAD_FP32;
 }
 
-// The list walk (listed.cuh) takes every AUTO launch once the neighbour lists
-// are built, whatever the autotuner chose among the tree kernels (4.9 times
-// faster at 1M rays, twice at 300).  Building them costs about 3 ns a point and
-// the allocation of 1 KB a point (2M points: 7 ms), a crossing on the tree 0.9 ns
-// (1M rays) to 6 ns (16,384 rays), so they are built when the crossings walked on
-// the cloud without them, 1.5 cube roots of n a ray, reach the number of points:
-// a cloud that sees a few rays never pays for them.
-constexpr double kNbrCrossingsPerPoint = 1.0;
+// What a crossing costs more on the tree than on the lists, in ns, by the launch's
+// rays: the smaller of the differences measured on uniform clouds of 20,000 to 2M
+// and clustered clouds of 500,000 to 16M points (tree / lists, uniform 100,000: 57 /
+// 14 at 289 rays, 14.5 / 4.2 at 1,024, 7.3 / 1.7 at 4,096, 5.7 / 0.6 at 16,384, 1.7 /
+// 0.25 at 65,536, 0.94 / 0.16 at 262,144, 0.60 / 0.11 at 1M).
+static double list_gain_ns(uint64_t nrays) {
+  constexpr double rays[] = {300, 1024, 4096, 16384, 65536, 262144, 1048576};
+  constexpr double ns[] = {36, 10, 5, 4, 1.7, 0.7, 0.4};
+  const double m = (double)nrays;
+  if (m <= rays[0]) return ns[0];
+  for (int i = 1; i < 7; ++i)
+    if (m < rays[i]) {
+      const double t = std::log(m / rays[i - 1]) / std::log(rays[i] / rays[i - 1]);
+      return ns[i - 1] * std::pow(ns[i] / ns[i - 1], t);
+    }
+  return ns[6];
+}
+// Building and later freeing the lists, with their records: 0.9 to 1.2 ms for
+// 20,000 and 100,000 points, 6 for 2M, 37 to 41 for 16M.
+static double list_cost_ns(uint64_t npart) { return 1.0e6 + 2.5 * (double)npart; }
+
+// AUTO.  The lists are built when the time that they would have saved so far, the
+// coming call included and with 1.5 cube roots of n crossings a ray, reaches what they
+// cost: a cloud that sees a few rays never pays for them.  (Below 8,192 points, where
+// the cost is three allocations whatever the size and two or three calls pay it back,
+// when the crossings reach the number of points.)  From then on the list
+// walk takes the launches, unless its last one asked the tree more than once in 12
+// crossings.  Asks cost several tree queries each (few lanes of a warp run them):
+// clustered clouds of 20,000 points ask at 0.47 of the crossings and are 2 times
+// slower on the lists at 1,024 rays and 1.1 at 262,144, 100,000 points at 0.17 (1.4
+// times slower, 1.2 faster), 500,000 points at 0.07 (1.2 and 1.9 faster).  There both
+// walks are timed by launch size, twice each (the list walk once where it asks at a
+// quarter of the crossings), and the faster one is taken; one in 32 launches tries the
+// list walk again.  The rays of these launches may differ: times are per crossing.
+constexpr double kListAskShare = 1.0 / 12.0;
+constexpr unsigned kListRetry = 32;
+static bool list_chosen(vt_cloud* cl, uint64_t nrays) {
+  if (!cl->view.nbr) return false;
+  if (!(cl->list_ask_share > kListAskShare)) return true;
+  vt_cloud::AutoCost& a = cl->auto_cost[63 - __builtin_clzll(nrays | 1)];
+  if (a.runs[1] < (cl->list_ask_share > 0.25 ? 1 : 2)) return true;
+  if (a.runs[0] < 2) return false;
+  if (++a.calls % kListRetry == 0) return true;
+  return a.ns[1] <= a.ns[0];
+}
 int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
+  cl->auto_walk = -1;
   if (kernel != VT_KERNEL_AUTO) return kernel == kKernelList ? VT_KERNEL_BATCHED_FP64 : kernel;
   // (squares of distances above 1e16 do not leave FP32 much room)
   double extent = 0.0;
   for (int d = 0; d < 3; ++d) extent = fmax(extent, cl->view.bbhi[d] - cl->view.bblo[d]);
   if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64 && extent <= 1e16 &&
       cl->list_bytes != 0) {
-    cl->nbr_credit += 1.5 * std::cbrt((double)cl->npart) * (double)nrays;
-    if (cl->nbr_credit >= kNbrCrossingsPerPoint * (double)cl->npart) {
+    const bool small = cl->npart < 8192;
+    cl->nbr_credit += 1.5 * std::cbrt((double)cl->npart) * (double)nrays *
+                      (small ? 1.0 : list_gain_ns(nrays));
+    if (cl->nbr_credit >= (small ? (double)cl->npart : list_cost_ns(cl->npart))) {
       WalkIO io{};
       io.nrays = (int64_t)nrays;
       const int rc = build_nbr_lists(cl, list_scratch(cl, io) * sizeof(WalkRec));
@@ -122,7 +165,23 @@ int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
       if (!cl->view.nbr) cl->nbr_credit = 0.0;  // no room: not at every call
     }
   }
-  return cl->view.nbr ? kKernelList : resolve_tree_kernel(cl, nrays);
+  const bool list = list_chosen(cl, nrays);
+  cl->auto_walk = list ? 1 : 0;
+  return list ? kKernelList : resolve_tree_kernel(cl, nrays);
+}
+
+// Time and asks of a launch that AUTO chose, for the choices after it.
+void vt::note_walk(vt_cloud* cl, const DevStats& hs, float ms, int64_t nrays) {
+  const int w = cl->auto_walk;
+  if (w < 0 || !(ms > 0.f) || hs.crossings == 0 || nrays <= 0) return;
+  if (w == 1)
+    cl->list_ask_share =
+        hs.queries > 2 * hs.rays ? (double)(hs.queries - 2 * hs.rays) / (double)hs.crossings : 0.0;
+  vt_cloud::AutoCost& a = cl->auto_cost[63 - __builtin_clzll((unsigned long long)nrays)];
+  const float ns = ms * 1e6f / (float)hs.crossings;
+  // (a first launch may have waited for its code: the smaller of two)
+  a.ns[w] = a.runs[w] == 0 ? ns : (a.runs[w] == 1 ? fminf(a.ns[w], ns) : 0.5f * (a.ns[w] + ns));
+  if (a.runs[w] < 2) ++a.runs[w];
 }
 
 static cudaStream_t pick_stream(vt_cloud* cl, void* s) {
@@ -899,6 +958,7 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
   std::lock_guard<std::mutex> lk(cl->mu);
   VT_CUDA(cudaSetDevice(cl->device));
   if (nrays == 0) return set_error(VT_ERR_INVALID, "autotune needs at least one ray");
+  cl->auto_walk = -1;
   // the sample must fill the device several times over (148 SMs x 9 blocks
   // x 128 threads ~ 170K rays resident), or it favours configurations that
   // cope with low occupancy; with 2^20 rays it also runs the guarded-FP32

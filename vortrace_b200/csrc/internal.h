@@ -123,7 +123,16 @@ struct vt_cloud {
   vt::DevBuf<float4> leaf32_d;  // SoA leaf blocks (common.cuh)
   vt::DevBuf<float4> nbr_d;     // neighbour lists (nbrlist.cu) ...
   vt::DevBuf<uint32_t> nbr_hdr_d;
-  double nbr_credit = 0.0;      // ... and the crossings walked without them
+  double nbr_credit = 0.0;      // ... and the ns that they would have saved so far
+  double list_ask_share = 0.0;  // tree queries per crossing of the last list walk
+  // ns per crossing of AUTO's launches on the tree [0] and the lists [1], by the
+  // binary logarithm of their rays
+  struct AutoCost {
+    float ns[2] = {0.f, 0.f};
+    uint8_t runs[2] = {0, 0};
+    unsigned calls = 0;
+  } auto_cost[64];
+  int auto_walk = -1;  // the walk in progress: 0, 1 as above, -1 not AUTO's choice
   int64_t list_bytes = -1;      // most bytes they and a launch's records may take
   uint64_t list_gen = 0;        // bumped when they are freed
   // reference-order tree (tietree.cu), built when an exact tie needs it
@@ -196,6 +205,8 @@ int check_projectable(const vt_cloud* cl, int mode);
 int resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays);
 // the same without the list walk
 int resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays);
+// what a finished launch tells the next choices (ms 0: not timed)
+void note_walk(vt_cloud* cl, const DevStats& hs, float ms, int64_t nrays);
 // resident blocks per SM the launch bounds of the walk kernel that runs a
 // launch of nrays rays are compiled for (VT_KERNEL_THREAD_FP32,
 // _BATCHED_FP64, _BATCHED on the current device; 0 for the others)

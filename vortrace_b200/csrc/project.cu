@@ -211,6 +211,7 @@ static int run_walk_on(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int ker
 static int finish_walk(vt_cloud* cl, WalkIO& io, const DevStats& hs, float ms, cudaStream_t st,
                        vt_stats* stats, WalkDiag* d_diag) {
   if (hs.rays > 0) cl->cross_per_ray = (double)hs.crossings / (double)hs.rays;
+  note_walk(cl, hs, ms, io.nrays);
   if (stats) {
     stats->rays = hs.rays;
     stats->crossings = hs.crossings;
@@ -563,6 +564,7 @@ int run_walk(vt_cloud* cl, WalkIO& io, int out_kind, int mode, int kernel, cudaS
     if (cl->ws_rec.reserve(list_scratch(cl, io))) {
       cudaGetLastError();  // no memory for the boundaries: walk on the tree
       kernel = resolve_tree_kernel(cl, io.nrays);
+      cl->auto_walk = 0;
     }
     io.rec = cl->ws_rec.p;
   }

@@ -526,6 +526,8 @@ static int finish_tree(vt_cloud* cl, int depth, const double lo[3], const double
 
   drop_nbr_lists(cl);
   cl->nbr_credit = 0.0;
+  cl->list_ask_share = 0.0;
+  for (auto& a : cl->auto_cost) a = {};
   cl->perm_d = std::move(pa);
   cl->pts_d = std::move(pts);
   cl->pts32_d = std::move(pts32);
