@@ -364,10 +364,13 @@ void vt_graph_destroy(vt_graph *graph);
  *      kernel (its occupancy: all that its register cap lets fit, 3/4 or
  *      1/2 of them; a value above the cap of a later launch's kernel is
  *      clamped to that cap);
- *   3. with VT_PARAM_TUNE_LEAF_SIZE = 1, the tree's leaf size (the cloud's,
- *      6 and 12; each candidate rebuilds the tree, ~30 ms per 2M points,
- *      and the best one is kept, which invalidates graphs and tapes
- *      recorded before);
+ *   3. the list walk on the same tree, where the cloud may have lists (they
+ *      are built; leaves of more than 8 points and VT_PARAM_LIST_BYTES rule
+ *      them out);
+ *   4. with VT_PARAM_TUNE_LEAF_SIZE = 1, the tree's leaf size (the cloud's,
+ *      6 and 12; each candidate rebuilds the tree, ~20 ms per 2M points, and
+ *      the one with the fastest walk, tree or lists, is kept, which
+ *      invalidates graphs and tapes recorded before);
  * and makes the fastest the cloud's VT_KERNEL_AUTO choice for batches at
  * least as large as the sample (VT_PARAM_SMEM_LEVELS, VT_PARAM_BLOCKS_PER_SM
  * and VT_PARAM_LEAF_SIZE are set to its values).  The pending-point stack
@@ -375,14 +378,15 @@ void vt_graph_destroy(vt_graph *graph);
  * finished by the global-stack kernel.  Results of every configuration are
  * the same bits; only the speed changes. */
 typedef struct {
-  int32_t kernel;           /* chosen VT_KERNEL_*                            */
+  int32_t kernel;           /* the fastest tree kernel, VT_KERNEL_*          */
   int32_t smem_levels;      /* chosen tree levels in shared memory           */
-  int32_t tried;            /* configurations timed                          */
+  int32_t tried;            /* tree configurations timed                     */
   int32_t blocks_per_sm;    /* chosen resident blocks per SM (0: all fit)    */
   uint64_t sample_rays;     /* rays in the sample                            */
   double mcrossings_per_s;  /* the chosen configuration on the sample        */
   int32_t leaf_size;        /* the tree's leaf size after tuning             */
-  int32_t pad;
+  int32_t lists;            /* 1: the list walk is faster, AUTO runs it and  */
+                            /* not `kernel`                                  */
 } vt_tune_result;
 int vt_cloud_autotune(vt_cloud *cloud, const double *starts, const double *ends,
                       uint64_t nrays, int mode, uint64_t max_sample,

@@ -74,3 +74,19 @@ def test_clouds_that_lists_do_not_fit_go_back_to_the_tree():
     # tried, left after one or two launches, tried again once in 32
     assert walks.count("list") <= 4 and walks[first + 2: first + 20] == ["tree"] * 18
     assert "list" in walks[first + 20:]
+
+
+@pytest.mark.parametrize("kind,n,k,lists", [("uniform", 360_000, 180, True),
+                                            ("clustered", 20_000, 32, False)])
+@pytest.mark.parametrize("leaf_size", [False, True])
+def test_autotune_takes_the_faster_walk(kind, n, k, lists, leaf_size):
+    """360,000 points in leaves of up to 12 (more than 8 of them) can have no lists:
+    a leaf size that wins among the tree kernels must not keep them away."""
+    s, e = _grid(k, *((0, 100) if kind == "uniform" else (40, 60)))
+    pc = _cloud(kind, n)
+    pc.kernel = "plain"
+    want = pc.projection(s, e)
+    pc.kernel = "auto"
+    res = pc.autotune(s, e, leaf_size=leaf_size)
+    assert res["lists"] == lists and res["kernel"] in ("thread_fp32", "batched_fp64", "batched")
+    assert _walks(pc, s, e, want, 4) == ["list" if lists else "tree"] * 4

@@ -75,13 +75,13 @@ class TuneResult(C.Structure):
     _fields_ = [("kernel", C.c_int32), ("smem_levels", C.c_int32), ("tried", C.c_int32),
                 ("blocks_per_sm", C.c_int32), ("sample_rays", C.c_uint64),
                 ("mcrossings_per_s", C.c_double), ("leaf_size", C.c_int32),
-                ("pad", C.c_int32)]
+                ("lists", C.c_int32)]
 
     def as_dict(self):
         names = {v: k for k, v in KERNELS.items()}
         return {"kernel": names.get(self.kernel, self.kernel), "smem_levels": self.smem_levels,
                 "blocks_per_sm": self.blocks_per_sm, "leaf_size": self.leaf_size,
-                "tried": self.tried, "sample_rays": self.sample_rays,
+                "lists": bool(self.lists), "tried": self.tried, "sample_rays": self.sample_rays,
                 "mcrossings_per_s": self.mcrossings_per_s}
 
 

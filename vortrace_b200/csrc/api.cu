@@ -146,26 +146,36 @@ static bool list_chosen(vt_cloud* cl, uint64_t nrays) {
   if (++a.calls % kListRetry == 0) return true;
   return a.ns[1] <= a.ns[0];
 }
+// Whether a cloud may have lists (squares of distances above 1e16 do not leave FP32
+// much room).
+static bool list_eligible(const vt_cloud* cl) {
+  double extent = 0.0;
+  for (int d = 0; d < 3; ++d) extent = fmax(extent, cl->view.bbhi[d] - cl->view.bblo[d]);
+  return !cl->periodic && cl->view.leaf32 && cl->npart >= 64 && extent <= 1e16 &&
+         cl->list_bytes != 0;
+}
+// ... built with room for the records of launches over nrays rays, where there is room
+static int list_build(vt_cloud* cl, uint64_t nrays) {
+  WalkIO io{};
+  io.nrays = (int64_t)nrays;
+  return vt::build_nbr_lists(cl, vt::list_scratch(cl, io) * sizeof(WalkRec));
+}
 int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
   cl->auto_walk = -1;
   if (kernel != VT_KERNEL_AUTO) return kernel == kKernelList ? VT_KERNEL_BATCHED_FP64 : kernel;
-  // (squares of distances above 1e16 do not leave FP32 much room)
-  double extent = 0.0;
-  for (int d = 0; d < 3; ++d) extent = fmax(extent, cl->view.bbhi[d] - cl->view.bblo[d]);
-  if (!cl->periodic && !cl->view.nbr && cl->view.leaf32 && cl->npart >= 64 && extent <= 1e16 &&
-      cl->list_bytes != 0) {
+  const bool tuned = cl->tuned_list != 0 && nrays >= cl->tuned_min_rays;
+  if (tuned && cl->tuned_list < 0) return resolve_tree_kernel(cl, nrays);
+  if (!cl->view.nbr && list_eligible(cl)) {
     const bool small = cl->npart < 8192;
     cl->nbr_credit += 1.5 * std::cbrt((double)cl->npart) * (double)nrays *
                       (small ? 1.0 : list_gain_ns(nrays));
     if (cl->nbr_credit >= (small ? (double)cl->npart : list_cost_ns(cl->npart))) {
-      WalkIO io{};
-      io.nrays = (int64_t)nrays;
-      const int rc = build_nbr_lists(cl, list_scratch(cl, io) * sizeof(WalkRec));
+      const int rc = list_build(cl, nrays);
       if (rc) return resolve_tree_kernel(cl, nrays);
       if (!cl->view.nbr) cl->nbr_credit = 0.0;  // no room: not at every call
     }
   }
-  const bool list = list_chosen(cl, nrays);
+  const bool list = tuned ? cl->view.nbr != nullptr : list_chosen(cl, nrays);
   cl->auto_walk = list ? 1 : 0;
   return list ? kKernelList : resolve_tree_kernel(cl, nrays);
 }
@@ -1014,7 +1024,11 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
   struct Best {
     int kernel, smem, blocks;
     double ms;
-  } best{cands[0].kernel, cands[0].smem, 0, -1.0};
+    double list_ms;  // the list walk on the same tree (infinite: none)
+    double fastest() const { return fmin(ms, list_ms); }
+  };
+  constexpr double kNone = std::numeric_limits<double>::infinity();
+  Best best{cands[0].kernel, cands[0].smem, 0, -1.0, kNone};
   // 1. kernel (rays per warp) x shared-memory tree depth, all blocks that fit
   auto tune_kernel = [&]() -> int {
     best.ms = -1.0;
@@ -1023,7 +1037,7 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
       double ms = 0.0;
       const int r = time_cfg(cd.kernel, cd.smem, 0, ms);
       if (r) return r;
-      if (best.ms < 0.0 || ms < best.ms) best = Best{cd.kernel, cd.smem, 0, ms};
+      if (best.ms < 0.0 || ms < best.ms) best = Best{cd.kernel, cd.smem, 0, ms, kNone};
     }
     // 2. occupancy of the persistent kernel: fewer resident blocks than its
     // launch bounds allow (3/4 and 1/2 of them) leave each more L1
@@ -1033,10 +1047,23 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
       double ms = 0.0;
       const int r = time_cfg(best.kernel, best.smem, blocks, ms);
       if (r) return r;
-      if (ms < best.ms) best = Best{best.kernel, best.smem, blocks, ms};
+      if (ms < best.ms) best = Best{best.kernel, best.smem, blocks, ms, kNone};
+    }
+    // 3. the list walk, where the tree's leaves and the memory allow lists
+    if (list_eligible(cl)) {
+      const int r = list_build(cl, m);
+      if (r) return r;
+    }
+    if (cl->view.nbr) {
+      double ms = 0.0;
+      const int r = time_cfg(vt::kKernelList, best.smem, best.blocks, ms);
+      if (r) return r;
+      --result->tried;  // (counts the configurations of the tree kernels)
+      best.list_ms = ms;
     }
     return VT_OK;
   };
+  const bool had_lists = cl->view.nbr != nullptr;
   auto restore = [&]() {
     cl->smem_levels = saved_smem;
     cl->blocks_per_sm = saved_blocks;
@@ -1045,8 +1072,8 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
     restore();
     return rc;
   }
-  // 3. leaf size (rebuilds the tree for each candidate; the results do not
-  // depend on it)
+  // 4. leaf size (rebuilds the tree for each candidate; the results do not
+  // depend on it): the one on which the faster of both walks is fastest
   int best_leaf = cl->leaf_size;
   if (cl->tune_leaf && !cl->periodic) {
     const int leaf0 = cl->leaf_size;
@@ -1070,7 +1097,7 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
         rebuild(leaf0);
         return rc;
       }
-      if (best.ms < overall.ms) {
+      if (best.fastest() < overall.fastest()) {
         overall = best;
         best_leaf = leaf;
       }
@@ -1085,12 +1112,20 @@ int vt_cloud_autotune(vt_cloud* cl, const double* starts, const double* ends, ui
   cl->blocks_per_sm = best.blocks;
   cl->tuned_kernel = best.kernel;
   cl->tuned_min_rays = m;
+  cl->tuned_list = best.list_ms < best.ms ? 1 : (best.list_ms < kNone ? -1 : 0);
+  if (cl->tuned_list > 0 && list_eligible(cl)) {  // (a rebuilt tree lost them)
+    if ((rc = list_build(cl, m))) return rc;
+  } else if (cl->tuned_list < 0 && !had_lists) {
+    vt::drop_nbr_lists(cl);
+  }
   result->kernel = best.kernel;
   result->smem_levels = best.smem;
   result->blocks_per_sm = best.blocks;
   result->leaf_size = best_leaf;
   result->sample_rays = m;
-  result->mcrossings_per_s = best.ms > 0.0 ? (double)crossings / (best.ms * 1e3) : 0.0;
+  result->lists = cl->tuned_list > 0;
+  result->mcrossings_per_s =
+      best.fastest() > 0.0 ? (double)crossings / (best.fastest() * 1e3) : 0.0;
   return VT_OK;
   VT_GUARD_END
 }

@@ -110,6 +110,7 @@ struct vt_cloud {
   int detailed_kernel = VT_KERNEL_AUTO;  // kernel of the detailed projection
   int tuned_kernel = VT_KERNEL_AUTO;    // vt_cloud_autotune's choice for AUTO
   uint64_t tuned_min_rays = 0;          // ... for batches at least this large
+  int tuned_list = 0;                   // ... where the lists were faster: 1, not: -1
   int tune_leaf = 0;                    // vt_cloud_autotune also tries leaf sizes
   uint64_t tree_gen = 0;                // bumped by every tree build or load
   // device tree (tree order)

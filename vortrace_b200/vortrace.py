@@ -484,12 +484,14 @@ class ProjectionCloud:
 
     def autotune(self, pos_start, pos_end, *, reduction="integrate",
                  max_sample: int = 1048576, leaf_size: bool = False) -> dict:
-        """Time the walk kernels (rays per warp), shared-memory tree depths and
-        resident blocks per SM on a sample of these rays (extension; not in
-        the reference) and make the fastest the ``'auto'`` configuration
-        for batches at least as large as the sample; with ``leaf_size`` the
-        tree is also rebuilt with leaf sizes 6 and 12 and the fastest kept.
-        Results do not change, only the speed.  Returns the choice."""
+        """Time the tree kernels (rays per warp), shared-memory tree depths and
+        resident blocks per SM and the walk on neighbour lists on a sample of
+        these rays (extension; not in the reference) and make the fastest the
+        ``'auto'`` configuration for batches at least as large as the sample;
+        with ``leaf_size`` the tree is also rebuilt with leaf sizes 6 and 12 and
+        the fastest kept.  Results do not change, only the speed.  Returns the
+        choice: ``lists`` tells whether ``'auto'`` runs on the lists; if not, it
+        runs ``kernel``."""
         mode = self._validate_reduction(reduction)
         S = self._prepare_array_for_backend(pos_start).reshape(-1, 3)
         E = self._prepare_array_for_backend(pos_end).reshape(-1, 3)
