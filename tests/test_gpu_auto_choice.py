@@ -90,3 +90,50 @@ def test_autotune_takes_the_faster_walk(kind, n, k, lists, leaf_size):
     res = pc.autotune(s, e, leaf_size=leaf_size)
     assert res["lists"] == lists and res["kernel"] in ("thread_fp32", "batched_fp64", "batched")
     assert _walks(pc, s, e, want, 4) == ["list" if lists else "tree"] * 4
+
+
+def _nested():
+    import vortrace_b200 as vt
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        pos = W.nested_cloud(20_000, 5)[0]
+        return vt.ProjectionCloud(pos, np.ones(len(pos)), boundbox=[0, 100.0] * 3)
+
+
+def test_clouds_of_compact_groups_start_on_the_tree():
+    """The lists of compact groups leave the long sides of the cells around them open,
+    which the lists themselves tell: 6 to 8 times slower at 16,384 rays.  A first call
+    (a series of snapshots makes no other) and a graph, whose launches are not timed,
+    go to the tree; lists are tried once and left."""
+    import torch
+    from vortrace_b200.graph import ProjectionGraph
+    s, e = _grid(128, 0, 100)
+    pc = _nested()
+    pc.kernel = "plain"
+    want = pc.projection(s, e)
+    pc = _nested()
+    g = ProjectionGraph(pc, torch.as_tensor(s, device="cuda"), torch.as_tensor(e, device="cuda"))
+    g.launch()
+    st = g.finish()
+    assert st["queries"] > 1.5 * st["crossings"]
+    np.testing.assert_array_equal(g.out.cpu().numpy().reshape(want.shape), want)
+    pc._cloud.neighbour_lists()  # (they were built)
+    pc = _nested()
+    walks = _walks(pc, s, e, want, 30)
+    assert walks[:2] == ["tree"] * 2 and walks.count("list") <= 2
+    S, E = _grid(128, 0, 100)
+    g = ProjectionGraph(pc, torch.as_tensor(S, device="cuda"), torch.as_tensor(E, device="cuda"))
+    g.launch()
+    st = g.finish()
+    assert st["queries"] > 1.5 * st["crossings"]
+
+
+def test_graph_on_a_cloud_that_lists_fit():
+    import torch
+    from vortrace_b200.graph import ProjectionGraph
+    s, e = _grid(128, 0, 100)
+    pc = _cloud("uniform", 20_000)
+    g = ProjectionGraph(pc, torch.as_tensor(s, device="cuda"), torch.as_tensor(e, device="cuda"))
+    g.launch()
+    st = g.finish()
+    assert st["queries"] < 0.5 * st["crossings"]

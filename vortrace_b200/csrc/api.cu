@@ -127,24 +127,41 @@ static double list_cost_ns(uint64_t npart) { return 1.0e6 + 2.5 * (double)npart;
 // cost: a cloud that sees a few rays never pays for them.  (Below 8,192 points, where
 // the cost is three allocations whatever the size and two or three calls pay it back,
 // when the crossings reach the number of points.)  From then on the list
-// walk takes the launches, unless its last one asked the tree more than once in 12
-// crossings.  Asks cost several tree queries each (few lanes of a warp run them):
-// clustered clouds of 20,000 points ask at 0.47 of the crossings and are 2 times
-// slower on the lists at 1,024 rays and 1.1 at 262,144, 100,000 points at 0.17 (1.4
-// times slower, 1.2 faster), 500,000 points at 0.07 (1.2 and 1.9 faster).  There both
-// walks are timed by launch size, twice each (the list walk once where it asks at a
-// quarter of the crossings), and the faster one is taken; one in 32 launches tries the
-// list walk again.  The rays of these launches may differ: times are per crossing.
+// walk takes the launches that fit it; for the others both walks are timed by launch
+// size, the one that is expected to be faster twice and the other once, and the
+// faster one is taken.  One in 32 launches tries the other again (one in 256 where it
+// took four times as long).  The rays of these launches may differ: times are per
+// crossing.
+//
+// Whether a launch fits is read from the lists (list_open_share, nbrlist.cu) and from
+// the asks of the last list walk (an ask costs several tree queries, as few lanes of a
+// warp run it).  Tree / list times at 1,024 to 65,025, and at 400,000 and 2M rays through
+// the dense part and the whole of clouds of 2,000 to 8M points:
+//   share up to 0.114   uniform; clustered from 700,000     1.2 to 26     2.2 to 6.6
+//   0.14 to 0.41        clustered 300,000 on, nested 4M     0.67 to 3.2   1.8 to 3.0
+//   0.51 to 0.85        clustered 20,000 and 100,000        0.33 to 2.1   0.98 to 1.9
+//                       nested 1M to 8M                     0.52 to 1.7   1.04 to 2.5
+//   0.88 and more       nested 20,000 to 300,000, filaments 0.13 to 2.3   0.57 to 1.6
 constexpr double kListAskShare = 1.0 / 12.0;
-constexpr unsigned kListRetry = 32;
-static bool list_chosen(vt_cloud* cl, uint64_t nrays) {
+constexpr double kListOpenFits = 0.12, kListOpenSmall = 0.4, kListOpenLarge = 0.85;
+constexpr uint64_t kListManyRays = 262144;
+static bool list_fits(const vt_cloud* cl, uint64_t nrays) {
+  return cl->list_ask_share <= kListAskShare &&
+         cl->list_open_share <= (nrays < kListManyRays ? kListOpenFits : kListOpenLarge);
+}
+// `replay`: for all launches of a graph, which are not timed
+static bool list_chosen(vt_cloud* cl, uint64_t nrays, bool replay) {
   if (!cl->view.nbr) return false;
-  if (!(cl->list_ask_share > kListAskShare)) return true;
+  if (list_fits(cl, nrays)) return true;
+  const int guess = cl->list_open_share <=
+                    (nrays < vt::kThreadKernelMinRays ? kListOpenSmall : kListOpenLarge);
   vt_cloud::AutoCost& a = cl->auto_cost[63 - __builtin_clzll(nrays | 1)];
-  if (a.runs[1] < (cl->list_ask_share > 0.25 ? 1 : 2)) return true;
-  if (a.runs[0] < 2) return false;
-  if (++a.calls % kListRetry == 0) return true;
-  return a.ns[1] <= a.ns[0];
+  if (!replay && a.runs[guess] < 2) return guess;
+  if (a.runs[0] == 0 || a.runs[1] == 0) return replay ? guess : !guess;
+  const bool list = a.ns[1] <= a.ns[0];
+  if (replay) return list;
+  const bool far = a.ns[list] * 4.f <= a.ns[!list];
+  return ++a.calls % (far ? 256 : 32) == 0 ? !list : list;
 }
 // Whether a cloud may have lists (squares of distances above 1e16 do not leave FP32
 // much room).
@@ -160,7 +177,7 @@ static int list_build(vt_cloud* cl, uint64_t nrays) {
   io.nrays = (int64_t)nrays;
   return vt::build_nbr_lists(cl, vt::list_scratch(cl, io) * sizeof(WalkRec));
 }
-int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
+int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays, bool replay) {
   cl->auto_walk = -1;
   if (kernel != VT_KERNEL_AUTO) return kernel == kKernelList ? VT_KERNEL_BATCHED_FP64 : kernel;
   const bool tuned = cl->tuned_list != 0 && nrays >= cl->tuned_min_rays;
@@ -175,7 +192,7 @@ int vt::resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays) {
       if (!cl->view.nbr) cl->nbr_credit = 0.0;  // no room: not at every call
     }
   }
-  const bool list = tuned ? cl->view.nbr != nullptr : list_chosen(cl, nrays);
+  const bool list = tuned ? cl->view.nbr != nullptr : list_chosen(cl, nrays, replay);
   cl->auto_walk = list ? 1 : 0;
   return list ? kKernelList : resolve_tree_kernel(cl, nrays);
 }

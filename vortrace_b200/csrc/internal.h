@@ -125,6 +125,7 @@ struct vt_cloud {
   vt::DevBuf<float4> nbr_d;     // neighbour lists (nbrlist.cu) ...
   vt::DevBuf<uint32_t> nbr_hdr_d;
   double nbr_credit = 0.0;      // ... and the ns that they would have saved so far
+  double list_open_share = 0.0;  // share of the cells' surface that they leave open
   double list_ask_share = 0.0;  // tree queries per crossing of the last list walk
   // ns per crossing of AUTO's launches on the tree [0] and the lists [1], by the
   // binary logarithm of their rays
@@ -154,7 +155,7 @@ struct vt_cloud {
   vt::DevBuf<vt::DevStats> ws_stats;
   vt::DevBuf<uint8_t> ws_tmp;
   vt::DevBuf<uint8_t> ws_order;  // ray sort keys, order and CUB scratch
-  vt::DevBuf<vt::WalkRec> ws_rec;  // boundaries of the list walk
+  vt::DevBuf<vt::WalkRec> ws_rec;  // records of the list walk
 };
 
 // Segment tape of one 'integrate' or 'volume' forward
@@ -202,8 +203,8 @@ int upload_fields(vt_cloud* cl, const double* src, bool src_device, cudaStream_t
 // tree built, mode valid, volume needs valid RGBA (src/reduction.cpp:59-66)
 int check_projectable(const vt_cloud* cl, int mode);
 // the kernel VT_KERNEL_AUTO stands for with this cloud and batch size
-// (builds the neighbour lists when they are due)
-int resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays);
+// (builds the neighbour lists when they are due); `replay`: for a graph's launches
+int resolve_kernel(vt_cloud* cl, int kernel, uint64_t nrays, bool replay = false);
 // the same without the list walk
 int resolve_tree_kernel(const vt_cloud* cl, uint64_t nrays);
 // what a finished launch tells the next choices (ms 0: not timed)

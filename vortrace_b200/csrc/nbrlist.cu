@@ -300,6 +300,71 @@ __global__ void __launch_bounds__(kNbrWarps * 32)
   }
 }
 
+// Sums over every `step`-th point and 32 directions u: sum[0] of s^2, s the extent of
+// the point's cell along u as its list has it (no farther than the cloud's box), the
+// weight with which rays meet this part of the cell; sum[1] of the s^2 whose end the
+// list does not vouch for (2 s > rho).  One warp per point, a direction per lane.
+__global__ void __launch_bounds__(128)
+    k_nbr_open(DevCloud c, int64_t step, double* __restrict__ sum) {
+  const int lane = threadIdx.x & 31;
+  const int64_t i = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * step;
+  if (i >= c.n) return;
+  const unsigned hdr = __ldg(&c.nbr_hdr[i]);
+  if (hdr == 0) return;
+  // a spiral of directions: equal steps in z, the golden angle around it
+  const float uz = 1.f - (float)(2 * lane + 1) / 32.f, ur = sqrtf(1.f - uz * uz);
+  float ux, uy;
+  sincosf(2.39996323f * (float)lane, &uy, &ux);
+  ux *= ur;
+  uy *= ur;
+  const double4 P = ldg_pt(&c.pts[i]);
+  auto side = [&](int d, double p, float u) {
+    return u == 0.f ? __int_as_float(0x7f800000)
+                    : (float)(((u > 0.f ? c.bbhi[d] : c.bblo[d]) - p) / (double)u);
+  };
+  float s = fminf(side(0, P.x, ux), fminf(side(1, P.y, uy), side(2, P.z, uz)));
+  const float* list = reinterpret_cast<const float*>(c.nbr) + i * (kNbrGroups * 16);
+  const int n_up = 4 * (int)((hdr >> 5) & 31u), n = n_up + 4 * (int)(hdr & 31u);
+  for (int k = 0; k < n; ++k) {
+    const int slot = k < n_up ? k : 4 * kNbrGroups - n + k;
+    const float* v = list + 16 * (slot >> 2) + (slot & 3);
+    const float x = __ldg(v), y = __ldg(v + 4), z = __ldg(v + 8);
+    const float den = x * ux + y * uy + z * uz;
+    if (den > 0.f) s = fminf(s, 0.5f * (x * x + y * y + z * z) / den);
+  }
+  const double w = (double)s * (double)s;
+  // hdr: rho^2 / 2
+  double all = w, open = 2.0 * w > (double)__uint_as_float(hdr & ~1023u) ? w : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    all += __shfl_xor_sync(kAll, all, o);
+    open += __shfl_xor_sync(kAll, open, o);
+  }
+  if (lane == 0) {
+    atomicAdd(&sum[0], all);
+    atomicAdd(&sum[1], open);
+  }
+}
+
+// The share of the cells' surface, as rays meet it, at which the lists cannot tell the
+// next cell: AUTO's measure of whether the list walk fits the cloud.  At most
+// kNbrOpenPoints of the points are looked at.
+constexpr int64_t kNbrOpenPoints = 65536;
+static int nbr_open_share(vt_cloud* cl, double& share) {
+  DevBuf<double> sum;
+  double h[2] = {0.0, 0.0};
+  if (sum.alloc(2)) return VT_ERR_NOMEM;
+  VT_CUDA(cudaMemsetAsync(sum.p, 0, 2 * sizeof(double), cl->stream));
+  const int64_t n = cl->view.n, step = (n + kNbrOpenPoints - 1) / kNbrOpenPoints;
+  const int64_t points = (n + step - 1) / step;
+  k_nbr_open<<<(unsigned)((points + 3) / 4), 128, 0, cl->stream>>>(cl->view, step, sum.p);
+  VT_CUDA(cudaGetLastError());
+  VT_CUDA(cudaMemcpyAsync(h, sum.p, sizeof(h), cudaMemcpyDeviceToHost, cl->stream));
+  VT_CUDA(cudaStreamSynchronize(cl->stream));
+  share = h[0] > 0.0 ? h[1] / h[0] : 1.0;
+  return VT_OK;
+}
+
 void drop_nbr_lists(vt_cloud* cl) {
   cl->nbr_d.reset();
   cl->nbr_hdr_d.reset();
@@ -335,10 +400,11 @@ int build_nbr_lists(vt_cloud* cl, size_t records) {
   k_nbr_lists<<<blocks, kNbrWarps * 32, 0, cl->stream>>>(cl->view, (float*)cl->nbr_d.p,
                                                          cl->nbr_hdr_d.p);
   VT_CUDA(cudaGetLastError());
-  VT_CUDA(cudaStreamSynchronize(cl->stream));
   cl->view.nbr = cl->nbr_d.p;
   cl->view.nbr_hdr = cl->nbr_hdr_d.p;
-  return VT_OK;
+  const int rc = nbr_open_share(cl, cl->list_open_share);
+  if (rc) drop_nbr_lists(cl);
+  return rc;
 }
 
 }  // namespace vt

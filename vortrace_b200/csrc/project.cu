@@ -674,7 +674,7 @@ int vt_graph_create(vt_cloud* cl, const double* d_starts, const double* d_ends, 
     io.gstack_s = g->stack_s.p;
     io.gstack_cap = cl->stack_cap;
     io.slow_threads = slow_threads;
-    int k = resolve_kernel(cl, kernel, nrays);
+    int k = resolve_kernel(cl, kernel, nrays, true);
     if (k == kKernelList) {
       if (g->rec.alloc(list_scratch(cl, io))) {
         cudaGetLastError();
