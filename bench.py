@@ -9,12 +9,11 @@ cloud and its device tree are built once, outside the timed region, as the
 reference's timing of Projection::makeProjection excludes buildTree).
 Prints one JSON line (rank 0).
 
-Metric: cell crossings per second (Mcrossings/s) of the batched kernel
-(VT_KERNEL_AUTO after vt_cloud_autotune on the workload's rays: persistent,
-one ray per thread in a coherent sorted order with the bounded guarded-FP32
-or FP64 k-NN, or one ray per warp for small batches), forward; the same
-line reports forward+adjoint, the bounded-FP64 variant of the batched
-kernel and the plain FP64 one-ray-per-thread kernel.  Multi-GPU (torchrun): every rank projects its own
+Metric: cell crossings per second (Mcrossings/s) of VT_KERNEL_AUTO after
+vt_cloud_autotune on the workload's rays (the walk on neighbour lists, or the
+faster of the tree kernels where the lists do not pay; `kernel` names the one
+that ran), forward; the same line reports forward+adjoint, the bounded-FP64
+variant of the batched tree kernel and the plain FP64 one-ray-per-thread kernel.  Multi-GPU (torchrun): every rank projects its own
 view of the cloud (the grid rotated about the cloud centre by 2*pi*rank/N):
 weak scaling, no data-path collective; value = all ranks' crossings / max
 over ranks of the timed device time.
@@ -51,14 +50,14 @@ BX = {"clustered_2m": 3262.25, "uniform_100k": 2915.74, "volume_2m": 3273.36,
 L2_FLUSH_BYTES = 256 << 20  # > 126 MB L2
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per crossing of
 # the walk kernel, from one single-pass ncu capture of the same launch
-# (clustered_2m, 1024x1024 rays, guarded-FP32 kernel at 9 blocks per SM with
-# 3 tree levels in shared memory, vortrace_b200.profile_walk: 63.70 GB read
-# + 66.01 GB written for 198,903,587 crossings; the writes are local memory,
-# as the image is 25 MB: the spill and stack slots of 170K resident threads
-# outgrow the L2), keyed by
-# (workload, AUTO kernel); other launches of the kernel are taken to scale
-# with their crossings.
-DRAM_BYTES_PER_CROSSING = {("clustered_2m", "thread_fp32"): 652.15}
+# (clustered_2m, 1024x1024 rays, 198,903,587 crossings, vortrace_b200.profile_walk).
+# List walk: 11.37 GB read (lists, points) + 4.25 GB written (records; the image is
+# 25 MB).  Guarded-FP32 kernel at 9 blocks per SM with 3 tree levels in shared memory:
+# 63.70 GB read + 66.01 GB written, local memory: the spill and stack slots of 170K
+# resident threads outgrow the L2.  Keyed by (workload, AUTO kernel); other launches
+# of the kernel are taken to scale with their crossings.
+DRAM_BYTES_PER_CROSSING = {("clustered_2m", "list"): 78.54,
+                           ("clustered_2m", "thread_fp32"): 652.15}
 
 
 def dist_env():
@@ -76,7 +75,7 @@ def host_cores():
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons sampled every 200 ms."""
+    """nvidia-smi clocks / throttle reasons sampled every 20 ms."""
 
     Q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
          "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -85,6 +84,7 @@ class ClockSampler:
     def __init__(self, gpu_index):
         self.idx = gpu_index
         self.lines = []
+        self.first = 0
         self.proc = None
         self.th = None
 
@@ -92,13 +92,18 @@ class ClockSampler:
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--query-gpu={self.Q}", "--format=csv,noheader,nounits",
-                 "-lms", "200", "-i", str(self.idx)], stdout=subprocess.PIPE,
+                 "-lms", "20", "-i", str(self.idx)], stdout=subprocess.PIPE,
                 stderr=subprocess.DEVNULL, text=True)
         except Exception:
             self.proc = None
             return
         self.th = threading.Thread(target=self._read, daemon=True)
         self.th.start()
+        # five steps take 0.16 s, nvidia-smi's start as long: samples count from here
+        t_end = time.monotonic() + 3.0
+        while not self.lines and time.monotonic() < t_end:
+            time.sleep(0.005)
+        self.first = len(self.lines)
 
     def _read(self):
         for line in self.proc.stdout:
@@ -116,7 +121,7 @@ class ClockSampler:
             self.th.join(timeout=5)
         sm, smax, reasons = [], 0.0, set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for ln in self.lines:
+        for ln in self.lines[self.first:] or self.lines:
             p = [x.strip() for x in ln.split(",")]
             if len(p) < 9:
                 continue
@@ -256,6 +261,36 @@ def oracle_sample_parity(w, pc, kernel, nsample=4096):
             "values_max_rel_err_vs_oracle": float(rel.max()) if rel.size else 0.0}, idx, o
 
 
+def roofline(name, kernel, crossings, launch_ms):
+    """Roofline of the walk kernel that ran (None where its bytes are not known).
+    Tree kernels: the algorithmic bytes of their searches.  The list walk makes no
+    searches: the DRAM bytes measured for its launch."""
+    listed = kernel == "list"
+    dpc = DRAM_BYTES_PER_CROSSING.get((name, kernel))
+    bx = dpc if listed else BX.get(name)
+    if not (bx and launch_ms):
+        return None
+    mp = os.path.join(ROOT, "MEASURED_PEAKS.json")
+    if os.path.exists(mp):
+        with open(mp) as f:
+            peak, peak_src = float(json.load(f)["hbm_gbs"]), "measured"
+    else:
+        peak, peak_src = 6650.0, "fallback"
+    achieved = crossings * bx / (launch_ms / 1e3) / 1e9
+    return {
+        "bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
+        "frac": round(achieved / peak, 4),
+        "traffic": round(dpc * crossings) if dpc else None,
+        "peak_source": peak_src, "bytes_per_crossing": bx,
+        "bytes": ("DRAM traffic of the launch, measured" if listed else
+                  "algorithmic bytes of the tree searches"),
+        "launch_ms": round(launch_ms, 3),
+        "kernel": {"list": "k_list (neighbour lists, coherent ray order)",
+                   "thread_fp32": "k_batched (guarded-FP32 k-NN, coherent ray order)",
+                   "batched_fp64": "k_batched (bounded FP64 k-NN, coherent ray order)",
+                   "batched": "k_warp (one ray per warp)"}.get(kernel, kernel)}
+
+
 def counters_run(w, kernel, tune, mode):
     """One forward of the guarded-FP32 kernel through the library built
     with the search counters (libvortrace_b200_counters.so), outside the
@@ -292,7 +327,8 @@ def counters_run(w, kernel, tune, mode):
     finally:
         lib.vt_cloud_destroy(h)
     q32 = max(1, st.fp32_queries)
-    return {"kernel": "k_batched guarded-FP32 (library built with VT_BATCHED_COUNTERS=1)",
+    return {"kernel": "k_batched guarded-FP32 (library built with VT_BATCHED_COUNTERS=1), "
+                      "whichever kernel was timed",
             "queries": int(st.queries), "fp32_split_queries": int(st.fp32_queries),
             "nodes_per_query": round(st.search_steps / max(1, st.queries), 3),
             "fp64_rechecks_per_query": round(st.fp64_checks / q32, 4),
@@ -424,10 +460,11 @@ def measure(name, args, rank, world, dev, K, W, *, kp=None, wp=None, full=True,
     # full size)
     tune = pc.autotune(S, E, reduction={L.REDUCE_VOLUME: "volume"}.get(mode, "integrate"),
                        max_sample=min(n, 1 << 20))
-    auto_kernel = tune["kernel"] if n >= tune["sample_rays"] else (
-        "batched" if n < 65536 else "thread_fp32")
+    # (the sample is never larger than the workload, so AUTO follows the result)
+    listed = bool(tune["lists"])
+    auto_kernel = "list" if listed else tune["kernel"]
 
-    # --- forward, batched kernel (the headline), clocks sampled meanwhile
+    # --- forward, AUTO (the headline), clocks sampled meanwhile
     for _ in range(W):
         fwd(L.KERNEL_AUTO)
     barrier()
@@ -500,33 +537,16 @@ def measure(name, args, rank, world, dev, K, W, *, kp=None, wp=None, full=True,
         "clocks": clocks,
     }
 
-    # --- roofline of the dominant kernel (k_batched + the tiny k_slow)
-    bx = BX.get(name)
-    mp = os.path.join(ROOT, "MEASURED_PEAKS.json")
-    if os.path.exists(mp):
-        with open(mp) as f:
-            peak, peak_src = float(json.load(f)["hbm_gbs"]), "measured"
-    else:
-        peak, peak_src = 6650.0, "fallback"
-    launch_ms = statistics.mean(walk_ms) if walk_ms else None
-    if bx and launch_ms:
-        achieved = crossings * bx / (launch_ms / 1e3) / 1e9
-        dpc = DRAM_BYTES_PER_CROSSING.get((name, auto_kernel))
-        rec["roofline"] = {
-            "bound": "hbm", "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
-            "frac": round(achieved / peak, 4),
-            "traffic": round(dpc * crossings) if dpc else None,
-            "peak_source": peak_src, "bytes_per_crossing": bx,
-            "launch_ms": round(launch_ms, 3),
-            "kernel": {"thread_fp32": "k_batched (guarded-FP32 k-NN, coherent ray order)",
-                       "batched_fp64": "k_batched (bounded FP64 k-NN, coherent ray order)",
-                       "batched": "k_warp (one ray per warp)"}.get(auto_kernel, auto_kernel)}
+    line = roofline(name, auto_kernel, crossings,
+                    statistics.mean(walk_ms) if walk_ms else None)
+    if line:
+        rec["roofline"] = line
 
     # --- parity (outside the timed region; one process: rank 0 of N = 1)
     if rank == 0 and world == 1:
         par = {"image_bit_identical_to_plain_fp64": bool(torch.equal(img_auto, img_plain))}
         try:
-            sp, idx, o = oracle_sample_parity(w, pc, auto_kernel)
+            sp, idx, o = oracle_sample_parity(w, pc, "auto" if listed else auto_kernel)
             par.update(sp)
             got = img_auto.cpu().numpy()[idx].reshape(len(idx), -1)
             par["image_rows_bit_identical_to_oracle"] = bool(np.array_equal(got, o))
@@ -629,8 +649,9 @@ def run_ours(args):
                 line[k] = rec[k]
         line.update({
             "e2e": e2e,
-            # per timed forward step: k_ray_keys, the walk kernel, k_slow, and
-            # for batches of fewer than 8 x 20 x 148 warps' rays also
+            # per timed forward step: k_ray_keys, the walk kernel, k_slow (the two
+            # launches over rays that the list walk left are not counted), and for
+            # batches of fewer than 8 x 20 x 148 warps' rays also
             # k_ray_cost, k_batch_keys and k_permute_batches (longest batches
             # first); CUB's radix-sort kernels not counted
             "gpu_launches": (3 + (3 if n < 8 * 20 * 148 * 32 else 0)) * K,
