@@ -55,8 +55,9 @@ extern "C" {
 #define VT_REDUCE_VOLUME 3
 
 /* ---- walk kernels ------------------------------------------------------ */
-#define VT_KERNEL_AUTO 0        /* one ray per thread on neighbour lists built  */
-                                /* on first need; before that and on trees with */
+#define VT_KERNEL_AUTO 0        /* one ray per thread on neighbour lists, built */
+                                /* when they pay, where they fit the cloud;     */
+                                /* before that, elsewhere and on trees with     */
                                 /* leaves of more than 8 points: THREAD_FP32,   */
                                 /* BATCHED below 65,536 rays, or the            */
                                 /* autotuner's choice.  Periodic clouds have one */

@@ -8,9 +8,10 @@
 //
 //   march   steps from cell to cell, each exit from the cell's neighbour list
 //           in FP32 coordinates relative to the cell, and records for every
-//           cell the boundary into it (t, in FP64) and whether the boundary is
-//           certified.  Where the list cannot tell, a tree query at the boundary
-//           point does;
+//           cell its line (the FP64 foot of its generator on the ray and the FP32
+//           squared offset, from which any two cells' boundary follows) and whether
+//           the boundary into it is certified.  Where the list cannot tell, a
+//           tree query at the boundary point does;
 //   replay  the reference's insertions (src/ray.cpp:187-430: the nearest cell of
 //           the split point of two pending cells) on the records alone: when
 //           every split point falls on one recorded cell, clear of its
@@ -63,12 +64,12 @@
 // boundary of adjacent cells it finds one of the two first, and accepts.
 //
 // The tree search of the other kernels costs 595 warp instructions per crossing;
-// this kernel takes 69 (clustered_2m, 512x512), and is bound by the latency of
-// dependent loads (8.6 of 13.4 cycles between two instructions of a warp): the
+// this kernel takes 68 (clustered_2m, 512x512), and is bound by the latency of
+// dependent loads (7.5 of 12.6 cycles between two instructions of a warp): the
 // lists (1 KB per point) and the records outgrow the L2.  Walk launch, tree
-// search -> lists: clustered_2m 1024x1024 171.6 -> 30.8 ms (march with its queries
+// search -> lists: clustered_2m 1024x1024 171.6 -> 31.1 ms (march with its queries
 // 20 ms, replay and walk 7, reduction 4.5), uniform_100k 128x128 6.3 -> 0.67 ms,
-// batched_1m 569 -> 166 ms (10 queries a ray outside the cloud).
+// batched_1m 569 -> 167 ms (10 queries a ray outside the cloud).
 #pragma once
 
 namespace vt {
@@ -380,10 +381,7 @@ __device__ __forceinline__ bool list_ends_clear(const WalkRec* rec, int n, doubl
 // certified, inserts and accepts exactly them: every split point it visits has to
 // fall on one cell clear of its neighbours (see the head of this file).  `gap`
 // bounds the difference of squared distances that counts as clear, `room` the
-// pending points; `depth` receives the most there were.  (A form in which the
-// warp replays a ray's disjoint stretches together on a copy in shared memory
-// was slower: 32.1 against 30.8 ms on clustered_2m, 189 against 166 ms on
-// batched_1m; the 25 KB a block are missing from the L1 of the march.)
+// pending points; `depth` receives the most there were.
 __device__ __forceinline__ bool list_replay(const WalkRec* rec, int n, double gap, int room,
                                          int& depth) {
   int stack[kBatchStack];
@@ -461,8 +459,8 @@ __global__ void __launch_bounds__(kListBlock, VT_LIST_MINB) k_list(DevCloud c, W
     };
 
     // ---- end cells and march.  A lane whose next step follows from its list
-    // goes on; the others' queries run together once they are half of the
-    // marching lanes.
+    // goes on; the others' queries run together once VT_LIST_WAIT or fewer lanes
+    // march for each of them.
     int phase = live ? 1 : 4;  // 1, 2: the ends' queries; 3: march; 4: through
     int c0 = -1;
     March m = {};

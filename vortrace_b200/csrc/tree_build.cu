@@ -210,7 +210,8 @@ __global__ void k_level_nodes(const double* __restrict__ x, const double* __rest
 // point and box side); here a level costs one bitonic sort in registers and shared
 // memory, one point to a thread, the segments side by side in slots of a power of
 // two.  Whole build, 1,000 / 20,000 / 1M / 2M points: 0.53 / 2.36 / 22.8 /
-// 29.3 -> 0.28 / 1.23 / 20.3 / 26.4 ms.
+// 29.3 -> 0.28 / 1.23 / 20.3 / 26.4 ms (with an allocation for each scratch array,
+// as it was then; build_tree_device has the times with one).
 constexpr int kTailSize = 1024;
 __global__ void __launch_bounds__(kTailSize)
     k_tail_levels(double* __restrict__ x, double* __restrict__ y, double* __restrict__ z,

@@ -8,7 +8,8 @@ Builds the workload's cloud (``vortrace_b200.workloads``), then runs
 device-resident rays and prints the crossings and the last launch's walk
 time.  No autotuning and no other kernel runs between the launches, so a
 profiler's ``-k regex:<kernel> -s <n> -c 1`` selects the (n+1)-th launch of
-that kernel.
+that kernel.  With ``--kernel auto`` the launches run on neighbour lists once they
+are built (``k_list``); ``--periodic`` makes the cloud periodic (``k_periodic``).
 """
 from __future__ import annotations
 
@@ -27,6 +28,7 @@ def main(argv=None):
     ap.add_argument("--smem-levels", type=int, default=3)
     ap.add_argument("--blocks-per-sm", type=int, default=0)
     ap.add_argument("--launches", type=int, default=5)
+    ap.add_argument("--periodic", action="store_true")
     a = ap.parse_args(argv)
 
     import torch
@@ -39,7 +41,8 @@ def main(argv=None):
     mode = {"integrate": L.REDUCE_SUM, "volume": L.REDUCE_VOLUME}[w["reduction"]]
     with warnings.catch_warnings():
         warnings.simplefilter("ignore")
-        pc = ProjectionCloud(w["pos"], w["fields"], boundbox=w["boundbox"])
+        pc = ProjectionCloud(w["pos"], w["fields"], boundbox=w["boundbox"],
+                             periodic=a.periodic)
     lib, h = pc._cloud._lib, pc._cloud._h
     pc._cloud.set_param(L.PARAM_SMEM_LEVELS, a.smem_levels)
     pc._cloud.set_param(L.PARAM_BLOCKS_PER_SM, a.blocks_per_sm)
@@ -55,7 +58,7 @@ def main(argv=None):
         L.check(lib.vt_project_device(h, d_s.data_ptr(), d_e.data_ptr(), n, mode,
                                       L.KERNELS[a.kernel], out.data_ptr(), stream, C.byref(st)))
     print(f"{a.config} npix={a.npix} kernel={a.kernel} rays={n} crossings={st.crossings} "
-          f"walk_ms={st.walk_ms:.3f}", flush=True)
+          f"queries={st.queries} walk_ms={st.walk_ms:.3f}", flush=True)
 
 
 if __name__ == "__main__":

@@ -6,8 +6,9 @@ as the reference; the work runs in libvortrace_b200.so (C ABI, ctypes) on a
 B200.  Extras that do not change the reference's calls:
   * ``kernel`` attribute: ``'auto'`` (one ray per thread on neighbour
     lists, which are built when the cloud has seen enough rays to pay for
-    them; before that the batched guarded-FP32 kernel, one ray per warp below
-    65,536 rays, or the autotuner's choice), ``'thread_fp32'``,
+    them, where they are the faster walk; else the batched guarded-FP32
+    kernel, one ray per warp below 65,536 rays, or the autotuner's choice),
+    ``'thread_fp32'``,
     ``'batched_fp64'``, ``'batched'`` (one ray per warp), ``'plain'`` (one ray
     per thread in the caller's order, FP64).  Periodic clouds have one kernel
     for all of these but ``'plain'``;
