@@ -404,7 +404,9 @@ int build_nbr_lists(vt_cloud* cl, size_t records) {
   cl->view.nbr_hdr = cl->nbr_hdr_d.p;
   const int rc = nbr_open_share(cl, cl->list_open_share);
   if (rc) drop_nbr_lists(cl);
-  return rc;
+  if (rc != VT_ERR_NOMEM) return rc;
+  cudaGetLastError();
+  return VT_OK;
 }
 
 }  // namespace vt
